@@ -110,29 +110,43 @@ def _heap(case):
     return tc.init(HEAP_BYTES)
 
 
+def _normal(seed):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    return lambda rows, cols, std=1.0: torch.empty(rows, cols, dtype=torch.bfloat16, device="cuda").normal_(0.0, std, generator=gen)
+
+
+def _gemm_inputs(case, normal):
+    return normal(case["m"], case["k"]), normal(case["n"], case["k"], 1.0 if case["op"] == "gemm_rs" else 0.02)
+
+
+def _mlp_inputs(case, normal):
+    """Activations, gate|up weight (128 gate rows, then the 128 up rows of the same features, and so on), down weight."""
+    h, f = case["hidden"], case["ffn"]
+    return normal(case["m"], h), normal(2 * f, h, 0.02), normal(h, f, 0.02)
+
+
 def prepare(case, seed):
     op, m = case["op"], case["m"]
-    gen = torch.Generator(device="cuda").manual_seed(seed)
-
-    def normal(rows, cols, std=1.0):
-        return torch.empty(rows, cols, dtype=torch.bfloat16, device="cuda").normal_(0.0, std, generator=gen)
-
+    normal = _normal(seed)
     if op == "silu_mul":
         gate_up = normal(m, 2 * case["ffn"])
         return _State(lambda: torch.ops.tileccl.silu_mul(gate_up), gate_up)
     heap = _heap(case)
     if op == "mlp":
         mlp = TpMlp(heap, m, case["hidden"], case["ffn"], seed=seed, graph=case["graph"])
-        mlp.x_shard.copy_(normal(m, case["hidden"]))
+        x, w_gate_up, w_down = _mlp_inputs(case, normal)
+        mlp.x_shard.copy_(x)
+        mlp.w_gate_up.copy_(w_gate_up)
+        mlp.w_down.copy_(w_down)
+        del x, w_gate_up, w_down
         if case["graph"]:
             mlp.capture()
         state = _State(mlp.replay if case["graph"] else mlp, mlp)
         _live.add(state)
         return state
-    n, k = case["n"], case["k"]
-    a, b_t = normal(m, k), normal(n, k, 1.0 if op == "gemm_rs" else 0.02)
+    a, b_t = _gemm_inputs(case, normal)
     if op == "ag_gemm_heap":
-        layer = AgGemm(heap, m, k, b_t, cta_group=2 if m % 256 == 0 else 1)
+        layer = AgGemm(heap, m, case["k"], b_t, cta_group=2 if m % 256 == 0 else 1)
         layer.a_shard.copy_(a)
         state = _State(layer, layer)
     else:
@@ -144,3 +158,22 @@ def prepare(case, seed):
 
 def run(state):
     return state.call()
+
+
+def exact(case, seed):
+    """The same pass in 64 bits, from the same inputs; none for results of over a gigabyte."""
+    op, normal = case["op"], _normal(seed)
+    if op == "silu_mul":
+        if case["m"] * case["ffn"] > 1 << 27:
+            return None
+        gate, up = normal(case["m"], 2 * case["ffn"]).double().split(case["ffn"], dim=1)
+        return gate * torch.sigmoid(gate) * up
+    if case["m"] * (case["hidden"] if op == "mlp" else case["n"]) > 1 << 27:
+        return None
+    if op == "mlp":
+        x, w_gate_up, w_down = _mlp_inputs(case, normal)
+        h = (x.double() @ w_gate_up.double().t()).view(case["m"], -1, 2, 128)
+        act = h[:, :, 0] * torch.sigmoid(h[:, :, 0]) * h[:, :, 1]
+        return act.reshape(case["m"], -1) @ w_down.double().t()
+    a, b_t = _gemm_inputs(case, normal)
+    return a.double() @ b_t.double().t()
