@@ -159,6 +159,13 @@ __device__ __forceinline__ uint32_t pack_bf16x2(uint32_t lo_f32_bits, uint32_t h
       : "f"(__uint_as_float(hi_f32_bits)), "f"(__uint_as_float(lo_f32_bits)));
   return r;
 }
+
+// silu(g) * u = g / (1 + exp(-g)) * u.  Written on exp(-|g|), so that the denominator lies in [1, 2]: there the
+// fast divide has no special range to lose, and gates below -88 (whose exp(-g) is infinite) keep their value.
+__device__ __forceinline__ float silu_mul_f32(float g, float u) {
+  const float e = __expf(-fabsf(g));
+  return __fdividef(g < 0.f ? g * e : g, 1.f + e) * u;
+}
 #endif  // __CUDACC__
 
 }  // namespace ptx
