@@ -1,0 +1,75 @@
+"""Tile widths of the GEMM kernel: every width and both CTA forms give the bits of the 256-column tile."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+WIDTHS = [32, 64, 96, 128, 160, 192, 224]
+
+
+def _operands(M, N, K, seed=0):
+    torch.manual_seed(M + N + K + seed)
+    return torch.randn(M, K, device="cuda", dtype=torch.bfloat16), torch.randn(N, K, device="cuda", dtype=torch.bfloat16) * 0.1
+
+
+def _same_as_reference(out, A, Bt):
+    ref = A.double() @ Bt.double().t()
+    # half a bf16 step, and K fp32 additions of terms of at most max|a| max|b|
+    tol = ref.abs() * 2.0 ** -8 + A.shape[1] * 2.0 ** -23 * float(A.abs().max()) * float(Bt.abs().max())
+    assert ((out.double() - ref).abs() <= tol).all()
+
+
+@pytest.mark.parametrize("cta_group", [1, 2])
+@pytest.mark.parametrize("width", WIDTHS)
+@pytest.mark.parametrize("store", ["st16", "st256"])
+def test_every_width_gives_the_same_bits(native_lib, cta_group, width, store):
+    from tileccl_b200.ops.gemm import GemmPlan
+    A, Bt = _operands(768, 1792, 1000)             # a K remainder, and a last tile that hangs over N for most widths
+    want = GemmPlan(A, Bt, cta_group=cta_group, tile_cols=256, timeout_ms=1000)
+    _same_as_reference(want(), A, Bt)
+    out = torch.full((769, 1792), 7.0, device="cuda", dtype=torch.bfloat16)
+    plan = GemmPlan(A, Bt, out=out[:768], cta_group=cta_group, tile_cols=width, store=store, timeout_ms=1000, num_ctas=10)
+    plan()
+    plan.check()
+    assert torch.equal(out[:768], want.out)
+    assert (out[768] == 7.0).all()
+
+
+@pytest.mark.parametrize("M", [128, 384, 1152])
+@pytest.mark.parametrize("width", [32, 160, 256])
+def test_pair_with_a_half_empty_last_tile(native_lib, M, width):
+    from tileccl_b200.ops.gemm import GemmPlan
+    A, Bt = _operands(M, 512, 328)
+    with pytest.raises(ValueError):
+        GemmPlan(A, Bt, cta_group=2)               # still refused unless asked for
+    out = torch.full((M + 256, 512), 7.0, device="cuda", dtype=torch.bfloat16)
+    plan = GemmPlan(A, Bt, out=out[:M], cta_group=2, ragged_m=True, tile_cols=width, timeout_ms=1000)
+    plan()
+    plan.check()
+    _same_as_reference(out[:M], A, Bt)
+    assert (out[M:] == 7.0).all()
+
+
+@pytest.mark.parametrize("cta_group", [1, 2])
+@pytest.mark.parametrize("width", WIDTHS)
+def test_gate_up_tiles_of_every_width(native_lib, cta_group, width):
+    from tileccl_b200.ops.gemm import GemmPlan
+    x, w = _operands(512, 2 * 640, 328)            # 640 features: a remainder for most widths
+    want = GemmPlan(x, w, cta_group=cta_group, epi="silu_mul", tile_cols=256, timeout_ms=1000)()
+    plan = GemmPlan(x, w, cta_group=cta_group, epi="silu_mul", tile_cols=width, timeout_ms=1000, num_ctas=6)
+    got = plan()
+    plan.check()
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("op", ["gemm", "gemm_rs", "ag_gemm"])
+@pytest.mark.parametrize("shape", [(128, 256, 64), (128, 2048, 520), (384, 768, 72), (640, 256, 8192), (2176, 3584, 256)])
+def test_ops_take_odd_multiples_of_128_rows(native_lib, op, shape):
+    import tileccl_b200 as tc
+    A, Bt = _operands(*shape)
+    tc.init(128 << 20)
+    try:
+        _same_as_reference(getattr(torch.ops.tileccl, op)(A, Bt), A, Bt)
+        tc.check_all()
+    finally:
+        tc.shutdown()

@@ -69,6 +69,8 @@ class GemmDesc(C.Structure):
         ("ag_vec32", C.c_int32),
         ("ag_warps", C.c_int32),
         ("epoch_dev", C.c_void_p),
+        ("ragged_m", C.c_int32),
+        ("tile_cols", C.c_int32),
     ]
 
 
@@ -118,6 +120,9 @@ def lib() -> C.CDLL:
     sig("tcl_gemm_plan_grid", i32, [vp])
     sig("tcl_gemm_plan_launches", i32, [vp])
     sig("tcl_gemm_smem_bytes", i32, [i32])
+    sig("tcl_gemm_pick_tile", i32, [i64, i64, i64, i32, i32, i32])
+    sig("tcl_gemm_pick_form", i32, [i64, i64, i64, i32])
+    sig("tcl_gemm_plan_tile_cols", i32, [vp])
     sig("tcl_sched_tile", None, [i32] * 8 + [C.POINTER(i32), C.POINTER(i32)])
     sig("tcl_barrier_all", i32, [C.POINTER(vp), i32, i32, i32, vp, u64, vp])
     sig("tcl_silu_mul", i32, [vp, vp, i64, i64, vp])

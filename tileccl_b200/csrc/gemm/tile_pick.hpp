@@ -1,0 +1,74 @@
+// Host rule that gives a GEMM its tile width (the columns of one scheduled tile).  Pure arithmetic, no CUDA
+// calls, so that it can be checked without a GPU.
+//
+// The accumulator rows of a tile are fixed (128 per CTA); its columns may be any multiple of 32 up to 256.  A
+// narrower tile reads more operand bytes per result, but lets a small problem reach more SMs, and lets a problem of
+// a few waves fill its last wave.  The estimate counts SM cycles, with constants measured on a B200 at 1965 MHz:
+//   a 64-deep k-block costs a CTA the longest of
+//     the tensor work (546 cycles at 256 columns),
+//     the issue loop of the producer (240 cycles and 45 for each TMA load: 64 to 160 columns take the same time), or of
+//     the MMA warp, which comes to the same with two loads,
+//     its share of what the L2 delivers to all active CTAs (10000 bytes a cycle, 95 to one CTA);
+//   128 columns of epilogue cost 1700 cycles; the epilogue of one tile overlaps the k-blocks of the next, the last
+//   one's is exposed; a CTA pair starts 2200 cycles later than a single CTA (cluster launch and barriers).
+// A narrower width has to gain more than kMargin: estimates closer than that came out either way from one board to the
+// next (512 x 8192 x 3584 in pairs: 224 columns 23.5 against 25.5 us on one, 28.1 against 24.8 us on another), and the wider tile reads less.
+// Device times in us, 256 columns against the width taken: 128 x 8192 x 3584 one-CTA 23.1 -> 15.3 (128 columns),
+// 384 x 3584 x 8192 47.5 -> 30.4 (128), 512 x 768 x 320 7.1 -> 5.5 (128), 2048 x 3584 x 8192 in pairs 111 -> 102 (224).
+#pragma once
+#include <cstdint>
+
+namespace tcl {
+
+constexpr int kMaxTileCols = 256;
+constexpr int kTileColStep = 32;      // cta_group::2 MMAs take N in steps of 32
+constexpr double kMargin = 0.10;
+
+// Rows of one TMA box of B: a CTA's whole share of a tile, or for a gate|up tile narrower than the weight's blocks of
+// 128 gate and 128 up rows the largest power of two in bn / 2, so that no box straddles two blocks.
+inline int b_box_rows(int cta_group, int bn, bool gate_up) {
+  if (!gate_up || bn == kMaxTileCols) return bn / cta_group;
+  int box = 128;
+  while ((bn / 2) % box != 0) box /= 2;
+  return box;
+}
+
+// Estimated SM cycles of an m x n x k GEMM in tiles of (128 * cta_group) x bn on `ctas` CTAs.
+inline double tile_cost(long long m, long long n, long long k, int cta_group, int ctas, int bn, bool gate_up) {
+  const long long kb = (k + 63) / 64;
+  const long long tiles = (m + 128 * cta_group - 1) / (128 * cta_group) * ((n + bn - 1) / bn);
+  const long long groups = ctas >= cta_group ? ctas / cta_group : 1;
+  const long long waves = (tiles + groups - 1) / groups;
+  const double active = static_cast<double>((tiles < groups ? tiles : groups) * cta_group);
+  const double bytes = 128.0 * 128.0 + 128.0 * bn / cta_group;      // per CTA and k-block
+  double block = bn * (546.0 / 256.0);
+  const double issue = 240.0 + 45.0 * (1 + bn / cta_group / b_box_rows(cta_group, bn, gate_up));
+  if (block < issue) block = issue;
+  if (block < bytes / 95.0) block = bytes / 95.0;
+  if (block < bytes * active / 10000.0) block = bytes * active / 10000.0;
+  const double main_loop = static_cast<double>(kb) * block;
+  const double epilogue = 1700.0 * ((bn + 127) / 128);
+  return static_cast<double>(waves) * (main_loop > epilogue ? main_loop : epilogue) + epilogue + (cta_group == 2 ? 2200.0 : 0.0);
+}
+
+// Columns per tile.
+inline int pick_tile_cols(long long m, long long n, long long k, int cta_group, int ctas, bool gate_up) {
+  int best = kMaxTileCols;
+  double cost = tile_cost(m, n, k, cta_group, ctas, best, gate_up);
+  for (int bn = kMaxTileCols - kTileColStep; bn >= kTileColStep; bn -= kTileColStep) {
+    const double c = tile_cost(m, n, k, cta_group, ctas, bn, gate_up);
+    if (c < cost * (1.0 - kMargin)) { best = bn; cost = c; }
+  }
+  return best;
+}
+
+// One CTA or a pair per tile, for rows that are a multiple of 128 (the pair's last tile may be half empty).  The pair
+// reads a third less from the L2; the single CTA starts earlier.  One-CTA against pair, us: 512 x 768 x 320 5.5 / 6.6,
+// 256 x 4096 x 4096 16.7 / 17.6, 512 x 8192 x 1024 11.2 / 12.2, 512 x 8192 x 3584 28.0 / 24.8, 4992 x 4096 x 4096 147 / 142.
+inline int pick_cta_group(long long m, long long n, long long k, int ctas) {
+  const double one = tile_cost(m, n, k, 1, ctas, pick_tile_cols(m, n, k, 1, ctas, false), false);
+  const double pair = tile_cost(m, n, k, 2, ctas, pick_tile_cols(m, n, k, 2, ctas, false), false);
+  return one < pair ? 1 : 2;
+}
+
+}  // namespace tcl

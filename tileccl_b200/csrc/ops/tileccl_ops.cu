@@ -9,6 +9,7 @@
 #include <new>
 
 #include "../gemm/gemm_sm100.cuh"
+#include "../gemm/tile_pick.hpp"
 
 namespace {
 
@@ -230,7 +231,7 @@ int tcl_gemm_desc_offset(const char* field) {
   TCL_OFF(mode) TCL_OFF(M) TCL_OFF(lda) TCL_OFF(A) TCL_OFF(world) TCL_OFF(seg_rows) TCL_OFF(dst_base) TCL_OFF(dst_row_off)
   TCL_OFF(rs_tile_cnt) TCL_OFF(rs_stage) TCL_OFF(rs_chunks) TCL_OFF(ag_src) TCL_OFF(ag_flags) TCL_OFF(gather_rows) TCL_OFF(ag_done)
   TCL_OFF(ag_push) TCL_OFF(ag_dst) TCL_OFF(barrier) TCL_OFF(status) TCL_OFF(timeout_ns) TCL_OFF(group_m) TCL_OFF(rs_mc_stage)
-  TCL_OFF(range_lo) TCL_OFF(epi_silu_mul) TCL_OFF(ablate) TCL_OFF(epi_st256) TCL_OFF(epi_tma_store) TCL_OFF(epoch_dev) TCL_OFF(ag_warps) TCL_OFF(rs_signal_batch) TCL_OFF(ag_vec32)
+  TCL_OFF(range_lo) TCL_OFF(epi_silu_mul) TCL_OFF(ablate) TCL_OFF(epi_st256) TCL_OFF(epi_tma_store) TCL_OFF(epoch_dev) TCL_OFF(ag_warps) TCL_OFF(ragged_m) TCL_OFF(tile_cols) TCL_OFF(rs_signal_batch) TCL_OFF(ag_vec32)
 #undef TCL_OFF
   return -1;
 }
@@ -238,6 +239,12 @@ int tcl_gemm_desc_offset(const char* field) {
 int tcl_gemm_smem_bytes(int cta_group) {
   return cta_group == 2 ? GemmCfg<2>::SMEM_BYTES : GemmCfg<1>::SMEM_BYTES;
 }
+
+int tcl_gemm_pick_tile(int64_t m, int64_t n, int64_t k, int cta_group, int ctas, int gate_up) {
+  return pick_tile_cols(m, n, k, cta_group, ctas, gate_up != 0);
+}
+int tcl_gemm_pick_form(int64_t m, int64_t n, int64_t k, int ctas) { return pick_cta_group(m, n, k, ctas); }
+int tcl_gemm_plan_tile_cols(void* plan) { return plan ? static_cast<GemmPlan*>(plan)->params.bn : 0; }
 
 void tcl_sched_tile(int m_tiles, int n_tiles, int group_m, int order, int world, int rank,
                     int rs_chunks, int t, int* m_blk, int* n_blk) {
@@ -250,7 +257,13 @@ void* tcl_gemm_plan_create(const tcl_gemm_desc* d, char* err, int errlen) {
   if (G != 1 && G != 2) { set_err(err, errlen, "cta_group must be 1 or 2"); return nullptr; }
   const int tile_m = 128 * G;
   if (d->M <= 0 || d->N <= 0 || d->K <= 0) { set_err(err, errlen, "M, N, K must be positive"); return nullptr; }
-  if (d->M % tile_m != 0) { set_err(err, errlen, "M must be a multiple of 128 * cta_group"); return nullptr; }
+  // ragged_m: the last pair's second half may lie below M (loaded as zeros, not stored)
+  if (d->ragged_m && (G != 2 || d->world != 1 || d->seg_rows != d->M || (d->mode == TCL_MODE_GEMM_RS && d->comm_enabled) || d->epi_tma_store)) {
+    set_err(err, errlen, "ragged_m needs cta_group 2, one row segment and no communication");
+    return nullptr;
+  }
+  const int m_step = d->ragged_m ? 128 : tile_m;
+  if (d->M % m_step != 0) { set_err(err, errlen, "M must be a multiple of 128 * cta_group"); return nullptr; }
   if (d->N % 256 != 0) { set_err(err, errlen, "N must be a multiple of 256"); return nullptr; }
   if (d->K % 8 != 0 || d->lda % 8 != 0 || d->ldb % 8 != 0 || d->ldc % 8 != 0) {
     set_err(err, errlen, "K and the row pitches must be multiples of 8 elements (16 bytes)");
@@ -264,7 +277,7 @@ void* tcl_gemm_plan_create(const tcl_gemm_desc* d, char* err, int errlen) {
     set_err(err, errlen, "world must be 1..8 and rank inside it");
     return nullptr;
   }
-  if (d->seg_rows <= 0 || d->seg_rows % tile_m != 0 || d->M % d->seg_rows != 0 ||
+  if (d->seg_rows <= 0 || d->seg_rows % m_step != 0 || d->M % d->seg_rows != 0 ||
       d->M / d->seg_rows > TCL_MAX_WORLD) {
     set_err(err, errlen, "seg_rows must divide M into at most 8 segments of whole tiles");
     return nullptr;
@@ -329,13 +342,34 @@ void* tcl_gemm_plan_create(const tcl_gemm_desc* d, char* err, int errlen) {
   p.status = d->status;
   p.timeout_ns = d->timeout_ns ? d->timeout_ns : 4000000000ull;
 
+  auto fail = [&](const char* m) -> void* { set_err(err, errlen, m); delete pl; return nullptr; };
+  int dev = 0, sms = 0;
+  const bool have_device = cudaGetDevice(&dev) == cudaSuccess &&
+                           cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0;
+  int grid = d->num_ctas > 0 ? d->num_ctas : sms;
+  if (grid > sms) grid = sms;
+
+  // The width is free where a tile is nobody else's unit: not across ranks (counters and reduce warps take 128 x 256
+  // tiles), not with the TMA-store epilogue (its boxes are 64 columns wide and would run over the next tile).
+  const bool local = d->world == 1 && !(d->mode == TCL_MODE_GEMM_RS && d->comm_enabled) && !d->epi_tma_store;
+  p.bn = local ? pick_tile_cols(d->M, d->N, d->K, G, grid, d->epi_silu_mul != 0) : kMaxTileCols;
+  if (d->tile_cols) {
+    if (d->tile_cols < kTileColStep || d->tile_cols > kMaxTileCols || d->tile_cols % kTileColStep != 0 || (!local && d->tile_cols != kMaxTileCols))
+      return fail("tile_cols must be a multiple of 32 up to 256, and 256 across ranks and with epi_tma_store");
+    p.bn = d->tile_cols;
+  }
+  p.b_gate_up = d->epi_silu_mul && p.bn < kMaxTileCols;
+  p.b_box = b_box_rows(G, p.bn, d->epi_silu_mul != 0);
+  p.b_loads = p.bn / G / p.b_box;
+  p.stage_bytes = GemmCfg<1>::A_BYTES + p.bn / G * GemmCfg<1>::BK * 2;
+  p.stages = GemmCfg<1>::STAGE_POOL / p.stage_bytes;
+  if (p.stages > GemmCfg<1>::MAX_STAGES) p.stages = GemmCfg<1>::MAX_STAGES;
+
   TileSched& sc = p.sched;
-  sc.m_tiles = d->M / tile_m;
-  sc.n_tiles = d->N / 256;
+  sc.m_tiles = (d->M + tile_m - 1) / tile_m;
+  sc.n_tiles = (d->N + p.bn - 1) / p.bn;
   sc.world = 1; sc.rank = 0; sc.rs_chunks = 1; sc.order = kOrderPlain;
   sc.group_m = d->group_m > 0 ? d->group_m : (G == 2 ? 8 : 16);
-
-  auto fail = [&](const char* m) -> void* { set_err(err, errlen, m); delete pl; return nullptr; };
 
   if (d->mode == TCL_MODE_GEMM_RS) {
     if (nseg != d->world) return fail("GEMM+RS: M / seg_rows must equal world");
@@ -407,14 +441,9 @@ void* tcl_gemm_plan_create(const tcl_gemm_desc* d, char* err, int errlen) {
     p.comm_enabled = 0;
   }
 
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-    return fail("no CUDA device");
-  int grid = d->num_ctas > 0 ? d->num_ctas : sms;
-  if (grid > sms) grid = sms;
+  if (!have_device) return fail("no CUDA device");
   const int max_useful = sc.num_tiles() * G;
-  if (grid > max_useful && d->mode == TCL_MODE_PLAIN) grid = max_useful;
+  if (grid > max_useful && (d->mode == TCL_MODE_PLAIN || local)) grid = max_useful;
   grid -= grid % G;
   if (grid < G) return fail("grid too small");
   pl->grid = grid;
@@ -424,13 +453,12 @@ void* tcl_gemm_plan_create(const tcl_gemm_desc* d, char* err, int errlen) {
   pl->a_ptr = d->A;
   if ((G == 2 ? prepare_gemm<2>() : prepare_gemm<1>()) != cudaSuccess) return fail("cudaFuncSetAttribute (dynamic shared memory) failed");
 
-  const int box_b = 256 / G;
   int r = ptx::encode_tmap_bf16_k64(&pl->tmap_a, d->A, static_cast<uint64_t>(d->M),
                                     static_cast<uint64_t>(d->K), static_cast<uint64_t>(d->lda), 128);
   if (r != 0) return fail("cuTensorMapEncodeTiled failed for A");
   r = ptx::encode_tmap_bf16_k64(&pl->tmap_b, d->B, static_cast<uint64_t>(d->N),
                                 static_cast<uint64_t>(d->K), static_cast<uint64_t>(d->ldb),
-                                static_cast<uint32_t>(box_b));
+                                static_cast<uint32_t>(p.b_box));
   if (r != 0) return fail("cuTensorMapEncodeTiled failed for B");
   return pl;
 }
@@ -455,7 +483,7 @@ int tcl_gemm_plan_set_operands(void* plan, const void* A, const void* B) {
   if (ptx::encode_tmap_bf16_k64(&ta, A, static_cast<uint64_t>(pl->params.M), static_cast<uint64_t>(pl->params.K),
                                 static_cast<uint64_t>(pl->lda), 128) != 0 ||
       ptx::encode_tmap_bf16_k64(&tb, B, static_cast<uint64_t>(pl->params.N), static_cast<uint64_t>(pl->params.K),
-                                static_cast<uint64_t>(pl->ldb), static_cast<uint32_t>(256 / pl->cta_group)) != 0)
+                                static_cast<uint64_t>(pl->ldb), static_cast<uint32_t>(pl->params.b_box)) != 0)
     return static_cast<int>(cudaErrorInvalidValue);
   pl->tmap_a = ta;
   pl->tmap_b = tb;

@@ -71,6 +71,9 @@ typedef struct tcl_gemm_desc {
   int32_t* epoch_dev;    /* optional: two zeroed ints in device memory.  When set, the kernel takes the call number from
                             epoch_dev[0] + 1 (and advances it when the call ends) instead of the `epoch` argument of
                             tcl_gemm_plan_run, so that a captured CUDA graph can replay the launch */
+  int32_t ragged_m;      /* cta_group 2, one row segment, no communication: M may be any multiple of 128 (the last pair's
+                            second half lies below M; it is loaded as zeros and not stored) */
+  int32_t tile_cols;     /* tile width in columns (a multiple of 32 up to 256), 0 = by estimate */
 } tcl_gemm_desc;
 
 /* Layout check for bindings that restate the struct: its size, and the offset of the named field
@@ -93,6 +96,11 @@ int tcl_gemm_plan_set_operands(void* plan, const void* A, const void* B);
 void tcl_gemm_plan_destroy(void* plan);
 int tcl_gemm_plan_grid(void* plan);
 int tcl_gemm_smem_bytes(int cta_group);
+/* Tile width (columns) that a plan of this shape gets on `ctas` CTAs, the CTA form (1, or 2 with ragged_m where M is an odd
+ * multiple of 128) that the estimate prefers, and the width a plan has. */
+int tcl_gemm_pick_tile(int64_t m, int64_t n, int64_t k, int cta_group, int ctas, int gate_up);
+int tcl_gemm_pick_form(int64_t m, int64_t n, int64_t k, int ctas);
+int tcl_gemm_plan_tile_cols(void* plan);
 /* Number of kernels one run launches (for launch accounting). */
 int tcl_gemm_plan_launches(void* plan);
 

@@ -39,7 +39,7 @@ class AgGemm:
     def __init__(self, heap: SymmetricHeap, M: int, K: int, Bt: torch.Tensor, cta_group: int = 2,
                  gather_rows: int = 512, out: torch.Tensor | None = None, group_m: int = 0,
                  num_ctas: int = 0, comm_enabled: bool = True, timeout_ms: float = 4000.0, ablate: int = 0, transport: str = "pull", item_rows: int = 1, epi: str | None = None,
-                 device_epoch: bool = False, hold_operands: bool = True, gather_warps: int = 0, vec32: bool = False):
+                 device_epoch: bool = False, hold_operands: bool = True, gather_warps: int = 0, vec32: bool = False, ragged_m: bool = False):
         require_bf16_rowmajor(Bt, "Bt")
         self.heap = heap
         world, rank = heap.world, heap.rank
@@ -50,7 +50,7 @@ class AgGemm:
         if Bt.shape[1] != K:
             raise ValueError("Bt must be [N, K]")
         seg = M // world
-        if M % world or seg % (128 * cta_group):
+        if M % world or seg % (128 if ragged_m else 128 * cta_group):      # ragged_m: one rank only, see GemmPlan
             raise ValueError("M / world must be a multiple of 128 * cta_group")
         gather_rows = min(gather_rows, seg)
         self.a_full = heap.empty((M, K), torch.bfloat16)
@@ -100,6 +100,7 @@ class AgGemm:
         d.timeout_ns = int(timeout_ms * 1e6)
         d.group_m, d.num_ctas = group_m, num_ctas
         d.ablate = ablate
+        d.ragged_m = 1 if ragged_m else 0
         own = (out, self.a_full, self.flags, self.done, self.barrier)
         self.plan = Plan(d, keep_alive=((Bt,) + own) if hold_operands else own, device_epoch=device_epoch)
         self.gather_rows = gather_rows

@@ -24,6 +24,7 @@ from __future__ import annotations
 
 import torch
 
+from .. import _native
 from ..parallel.heap import SymmetricHeap
 from . import elementwise as ew
 from .ag_gemm import AgGemm
@@ -79,11 +80,24 @@ _lib.define("silu_mul(Tensor gate_up) -> Tensor")
 _lib.define("barrier() -> ()")
 
 
+def _form(m: int, n: int, k: int, world: int) -> dict:
+    """CTA form of a plan whose rank holds ``m`` rows.  One rank: whichever is estimated to be faster, the pair
+    also for an odd multiple of 128 rows (last tile half empty).  Several: the pair where its 256-row tiles fit."""
+    if _ctx["cta_group"] != 2 or m % 128:
+        return {"cta_group": 1}
+    if world > 1:
+        return {"cta_group": 2 if m % 256 == 0 else 1}
+    sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+    if _native.lib().tcl_gemm_pick_form(m, n, k, sms) == 1:
+        return {"cta_group": 1}
+    return {"cta_group": 2, "ragged_m": m % 256 != 0}
+
+
 def _gemm(a: torch.Tensor, b_t: torch.Tensor) -> torch.Tensor:
     k = _key("gemm", a, b_t)
     plan = _ctx["plans"].get(k)
     if plan is None:
-        plan = _ctx["plans"][k] = GemmPlan(a, b_t, cta_group=_ctx["cta_group"] if a.shape[0] % 256 == 0 else 1, hold_operands=False)
+        plan = _ctx["plans"][k] = GemmPlan(a, b_t, hold_operands=False, **_form(a.shape[0], *b_t.shape, world=1))
     else:
         plan.set_operands(a, b_t)
     return plan()
@@ -94,8 +108,7 @@ def _gemm_rs(a: torch.Tensor, b_t: torch.Tensor) -> torch.Tensor:
     op = _ctx["plans"].get(k)
     if op is None:
         h = heap()
-        g = _ctx["cta_group"] if (a.shape[0] // h.world) % 256 == 0 else 1
-        op = _ctx["plans"][k] = GemmRs(h, a, b_t, cta_group=g, hold_operands=False)
+        op = _ctx["plans"][k] = GemmRs(h, a, b_t, hold_operands=False, **_form(a.shape[0] // h.world, *b_t.shape, world=h.world))
     else:
         op.plan.set_operands(a, b_t)
     return op()
@@ -107,8 +120,7 @@ def _ag_gemm(a_shard: torch.Tensor, b_t: torch.Tensor, gather_rows: int = 512) -
     k = _key("ag_gemm", b_t, extra=(M, K, gather_rows))
     op = _ctx["plans"].get(k)
     if op is None:
-        g = _ctx["cta_group"] if a_shard.shape[0] % 256 == 0 else 1
-        op = _ctx["plans"][k] = AgGemm(h, M, K, b_t, cta_group=g, gather_rows=gather_rows, hold_operands=False)
+        op = _ctx["plans"][k] = AgGemm(h, M, K, b_t, gather_rows=gather_rows, hold_operands=False, **_form(a_shard.shape[0], *b_t.shape, world=h.world))
     else:
         op.plan.set_operands(op.a_full, b_t)
     if a_shard.data_ptr() != op.a_shard.data_ptr():
