@@ -35,6 +35,34 @@ def test_every_width_gives_the_same_bits(native_lib, cta_group, width, store):
     assert (out[768] == 7.0).all()
 
 
+@pytest.mark.parametrize("K", [64, 128, 256, 328, 512, 576, 1000])      # 1 to 16 k-blocks around the skew of 4
+@pytest.mark.parametrize("N", [256, 512, 768, 1792])                     # with and without a last single half
+@pytest.mark.parametrize("num_ctas", [2, 8, 10, 0])
+def test_wide_tiles_give_the_same_bits(native_lib, K, N, num_ctas):
+    from tileccl_b200.ops.gemm import GemmPlan
+    A, Bt = _operands(1152, N, K)
+    want = GemmPlan(A, Bt, cta_group=2, ragged_m=True, tile_cols=256, timeout_ms=1000)()
+    _same_as_reference(want, A, Bt)
+    out = torch.full((1153, N), 7.0, device="cuda", dtype=torch.bfloat16)
+    plan = GemmPlan(A, Bt, out=out[:1152], cta_group=2, ragged_m=True, tile_cols=512, timeout_ms=1000, num_ctas=num_ctas)
+    for _ in range(2):
+        plan()
+        plan.check()
+    assert torch.equal(out[:1152], want)
+    assert (out[1152] == 7.0).all()
+
+
+@pytest.mark.parametrize("num_ctas", [2, 6, 0])
+def test_wide_gate_up_tiles(native_lib, num_ctas):
+    from tileccl_b200.ops.gemm import GemmPlan
+    x, w = _operands(768, 2 * 896, 520)
+    want = GemmPlan(x, w, cta_group=2, epi="silu_mul", tile_cols=256, timeout_ms=1000)()
+    plan = GemmPlan(x, w, cta_group=2, epi="silu_mul", tile_cols=512, timeout_ms=1000, num_ctas=num_ctas)
+    got = plan()
+    plan.check()
+    assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("M", [128, 384, 1152])
 @pytest.mark.parametrize("width", [32, 160, 256])
 def test_pair_with_a_half_empty_last_tile(native_lib, M, width):

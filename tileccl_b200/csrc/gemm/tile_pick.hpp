@@ -71,4 +71,27 @@ inline int pick_cta_group(long long m, long long n, long long k, int ctas) {
   return one < pair ? 1 : 2;
 }
 
+// Two adjacent 256-column tiles per work item (pair form only).  Large problems are bound by power: the tensor pipe is
+// active 92 % of the cycles, at whatever clock the power allows, so bytes not moved are time.  256 x 512 reads a quarter
+// less from the L2 than 256 x 256, but both accumulator buffers belong to one item and its epilogue is hidden only by
+// the skew at its ends.  Sustained, us, 256 against 512 columns: 8192^3 885 -> 843, 16384 x 7168 x 8192 1581 -> 1465,
+// 32768 x 28672 x 8192 13.3 -> 12.5 ms, 16384 x 8192 x 3584 758 -> 738, but K = 1024 (32768 x 8192) 453 -> 470, and with 2.2
+// waves of items (4992 x 4096 x 4096) 141 -> 145.
+constexpr int kWideMinK = 3072;
+constexpr int kWideMinWaves = 4;
+// Raster group of wide tiles, in tile rows: 16 x 256 rows by 4.6 x 512 columns is what 74 pairs work on at a time, nearer
+// to a square than with 8 rows (8192^3 846 -> 830 us, 16384 x 7168 x 8192 1515 -> 1458 us).
+constexpr int kWideGroupM = 16;
+
+inline bool pick_wide(long long m, long long n, long long k, int ctas) {
+  const long long pairs = ctas / 2;
+  return k >= kWideMinK && pairs > 0 && (m + 255) / 256 * ((n + 511) / 512) >= kWideMinWaves * pairs;
+}
+
+// Columns per work item: a tile's, or 512 for two of 256.
+inline int pick_cols(long long m, long long n, long long k, int cta_group, int ctas, bool gate_up) {
+  const int bn = pick_tile_cols(m, n, k, cta_group, ctas, gate_up);
+  return cta_group == 2 && bn == kMaxTileCols && pick_wide(m, n, k, ctas) ? 2 * kMaxTileCols : bn;
+}
+
 }  // namespace tcl

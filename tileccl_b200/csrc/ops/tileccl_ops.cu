@@ -241,10 +241,10 @@ int tcl_gemm_smem_bytes(int cta_group) {
 }
 
 int tcl_gemm_pick_tile(int64_t m, int64_t n, int64_t k, int cta_group, int ctas, int gate_up) {
-  return pick_tile_cols(m, n, k, cta_group, ctas, gate_up != 0);
+  return pick_cols(m, n, k, cta_group, ctas, gate_up != 0);
 }
 int tcl_gemm_pick_form(int64_t m, int64_t n, int64_t k, int ctas) { return pick_cta_group(m, n, k, ctas); }
-int tcl_gemm_plan_tile_cols(void* plan) { return plan ? static_cast<GemmPlan*>(plan)->params.bn : 0; }
+int tcl_gemm_plan_tile_cols(void* plan) { return plan ? static_cast<GemmPlan*>(plan)->params.bn * static_cast<GemmPlan*>(plan)->params.halves : 0; }
 
 void tcl_sched_tile(int m_tiles, int n_tiles, int group_m, int order, int world, int rank,
                     int rs_chunks, int t, int* m_blk, int* n_blk) {
@@ -352,24 +352,31 @@ void* tcl_gemm_plan_create(const tcl_gemm_desc* d, char* err, int errlen) {
   // The width is free where a tile is nobody else's unit: not across ranks (counters and reduce warps take 128 x 256
   // tiles), not with the TMA-store epilogue (its boxes are 64 columns wide and would run over the next tile).
   const bool local = d->world == 1 && !(d->mode == TCL_MODE_GEMM_RS && d->comm_enabled) && !d->epi_tma_store;
-  p.bn = local ? pick_tile_cols(d->M, d->N, d->K, G, grid, d->epi_silu_mul != 0) : kMaxTileCols;
+  const bool wide_ok = local && G == 2;
+  int cols = local ? pick_cols(d->M, d->N, d->K, G, grid, d->epi_silu_mul != 0) : kMaxTileCols;
   if (d->tile_cols) {
-    if (d->tile_cols < kTileColStep || d->tile_cols > kMaxTileCols || d->tile_cols % kTileColStep != 0 || (!local && d->tile_cols != kMaxTileCols))
-      return fail("tile_cols must be a multiple of 32 up to 256, and 256 across ranks and with epi_tma_store");
-    p.bn = d->tile_cols;
+    const bool legal = d->tile_cols == 2 * kMaxTileCols ? wide_ok
+                                                        : d->tile_cols >= kTileColStep && d->tile_cols <= kMaxTileCols && d->tile_cols % kTileColStep == 0;
+    if (!legal || (!local && d->tile_cols != kMaxTileCols))
+      return fail("tile_cols must be a multiple of 32 up to 256, or 512 in pairs, and 256 across ranks and with epi_tma_store");
+    cols = d->tile_cols;
   }
+  p.epi_warps = local && !d->epi_st256 && !d->ablate ? 8 : 4;
+  p.halves = cols > kMaxTileCols ? 2 : 1;
+  p.bn = cols / p.halves;
+  p.n_subs = (d->N + p.bn - 1) / p.bn;
   p.b_gate_up = d->epi_silu_mul && p.bn < kMaxTileCols;
   p.b_box = b_box_rows(G, p.bn, d->epi_silu_mul != 0);
   p.b_loads = p.bn / G / p.b_box;
-  p.stage_bytes = GemmCfg<1>::A_BYTES + p.bn / G * GemmCfg<1>::BK * 2;
+  p.stage_bytes = GemmCfg<1>::A_BYTES + p.halves * p.bn / G * GemmCfg<1>::BK * 2;
   p.stages = GemmCfg<1>::STAGE_POOL / p.stage_bytes;
   if (p.stages > GemmCfg<1>::MAX_STAGES) p.stages = GemmCfg<1>::MAX_STAGES;
 
   TileSched& sc = p.sched;
   sc.m_tiles = (d->M + tile_m - 1) / tile_m;
-  sc.n_tiles = (d->N + p.bn - 1) / p.bn;
+  sc.n_tiles = (d->N + cols - 1) / cols;
   sc.world = 1; sc.rank = 0; sc.rs_chunks = 1; sc.order = kOrderPlain;
-  sc.group_m = d->group_m > 0 ? d->group_m : (G == 2 ? 8 : 16);
+  sc.group_m = d->group_m > 0 ? d->group_m : p.halves == 2 ? kWideGroupM : (G == 2 ? 8 : 16);
 
   if (d->mode == TCL_MODE_GEMM_RS) {
     if (nseg != d->world) return fail("GEMM+RS: M / seg_rows must equal world");
@@ -382,7 +389,7 @@ void* tcl_gemm_plan_create(const tcl_gemm_desc* d, char* err, int errlen) {
     int g = d->rs_chunks > 0 ? d->rs_chunks : st;
     if (st % g != 0) return fail("GEMM+RS: rs_chunks must divide the tile rows of a segment");
     sc.rs_chunks = g;
-    if (d->group_m <= 0) {
+    if (d->group_m <= 0 && p.halves == 1) {
       const int per = 8 / d->world > 0 ? 8 / d->world : 1;
       sc.group_m = d->world * per;
     }
@@ -442,7 +449,16 @@ void* tcl_gemm_plan_create(const tcl_gemm_desc* d, char* err, int errlen) {
   }
 
   if (!have_device) return fail("no CUDA device");
-  const int max_useful = sc.num_tiles() * G;
+  p.items = p.wide_items = sc.num_tiles();
+  if (p.halves == 2) {
+    // the rest of the last wave goes out in halves where those fill at most one round of the grid
+    const int rest = sc.num_tiles() % (grid >= G ? grid / G : 1);
+    if (2 * rest <= grid / G) {
+      p.wide_items -= rest;
+      p.items += rest;
+    }
+  }
+  const int max_useful = p.items * G;
   if (grid > max_useful && (d->mode == TCL_MODE_PLAIN || local)) grid = max_useful;
   grid -= grid % G;
   if (grid < G) return fail("grid too small");

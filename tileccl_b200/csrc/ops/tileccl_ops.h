@@ -73,7 +73,7 @@ typedef struct tcl_gemm_desc {
                             tcl_gemm_plan_run, so that a captured CUDA graph can replay the launch */
   int32_t ragged_m;      /* cta_group 2, one row segment, no communication: M may be any multiple of 128 (the last pair's
                             second half lies below M; it is loaded as zeros and not stored) */
-  int32_t tile_cols;     /* tile width in columns (a multiple of 32 up to 256), 0 = by estimate */
+  int32_t tile_cols;     /* tile width in columns (a multiple of 32 up to 256, or 512 with cta_group 2), 0 = by estimate */
 } tcl_gemm_desc;
 
 /* Layout check for bindings that restate the struct: its size, and the offset of the named field

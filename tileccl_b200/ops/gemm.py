@@ -23,7 +23,7 @@ class GemmPlan(Plan):
         (cp.async.bulk.tensor stores from the staging buffer), the counterparts of the reference's
         direct-store and TMA-store epilogues (comm_comp/gemm_sm90.cuh:83-88).  ``ragged_m`` lets the CTA-pair form
         take an M that is an odd multiple of 128 (its last tile is half empty);
-        ``tile_cols`` fixes the width of a tile (a multiple of 32 up to 256; 0 = chosen for the shape)."""
+        ``tile_cols`` fixes the width of a tile (a multiple of 32 up to 256, or 512 in pairs; 0 = chosen for the shape)."""
         if store not in ("st16", "st256", "tma"):
             raise ValueError("store must be st16, st256 or tma")
         require_bf16_rowmajor(A, "A")
