@@ -43,7 +43,7 @@ cudaError_t prepare_gemm() {
 }
 
 template <int G>
-cudaError_t launch_gemm(const GemmPlan* pl, const GemmParams& params, cudaStream_t stream) {
+cudaError_t launch_gemm(const GemmPlan* pl, const CUtensorMap& tmap_a, const CUtensorMap& tmap_b, const GemmParams& params, cudaStream_t stream) {
   using Cfg = GemmCfg<G>;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(pl->grid), 1, 1);
@@ -57,7 +57,26 @@ cudaError_t launch_gemm(const GemmPlan* pl, const GemmParams& params, cudaStream
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, gemm_sm100_kernel<G>, pl->tmap_a, pl->tmap_b, params, pl->omaps);
+  return cudaLaunchKernelEx(&cfg, gemm_sm100_kernel<G>, tmap_a, tmap_b, params, pl->omaps);
+}
+
+// Tensor maps of other operands with the plan's shapes and row pitches.  0 or a CUDA error.
+int encode_operands(const GemmPlan* pl, const void* A, const void* B, CUtensorMap* ta, CUtensorMap* tb) {
+  if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return static_cast<int>(cudaErrorMisalignedAddress);
+  if (ptx::encode_tmap_bf16_k64(ta, A, static_cast<uint64_t>(pl->params.M), static_cast<uint64_t>(pl->params.K),
+                                static_cast<uint64_t>(pl->lda), 128) != 0 ||
+      ptx::encode_tmap_bf16_k64(tb, B, static_cast<uint64_t>(pl->params.N), static_cast<uint64_t>(pl->params.K),
+                                static_cast<uint64_t>(pl->ldb), static_cast<uint32_t>(pl->params.b_box)) != 0)
+    return static_cast<int>(cudaErrorInvalidValue);
+  return 0;
+}
+
+int run_plan(const GemmPlan* pl, const CUtensorMap& ta, const CUtensorMap& tb, int epoch, void* stream) {
+  // The call number travels in a copy of the parameters: a launch does not write to the plan.
+  GemmParams params = pl->params;
+  params.epoch = epoch;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  return static_cast<int>(pl->cta_group == 2 ? launch_gemm<2>(pl, ta, tb, params, st) : launch_gemm<1>(pl, ta, tb, params, st));
 }
 
 // ---------------------------------------------------------------------------
@@ -482,25 +501,26 @@ void* tcl_gemm_plan_create(const tcl_gemm_desc* d, char* err, int errlen) {
 int tcl_gemm_plan_run(void* plan, int epoch, void* stream) {
   GemmPlan* pl = static_cast<GemmPlan*>(plan);
   if (!pl) return static_cast<int>(cudaErrorInvalidValue);
-  // The call number travels in a copy of the parameters: a launch does not write to the plan.
-  GemmParams params = pl->params;
-  params.epoch = epoch;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  cudaError_t e = pl->cta_group == 2 ? launch_gemm<2>(pl, params, st) : launch_gemm<1>(pl, params, st);
-  return static_cast<int>(e);
+  return run_plan(pl, pl->tmap_a, pl->tmap_b, epoch, stream);
+}
+
+int tcl_gemm_plan_run_on(void* plan, const void* A, const void* B, int epoch, void* stream) {
+  GemmPlan* pl = static_cast<GemmPlan*>(plan);
+  if (!pl || !A || !B) return static_cast<int>(cudaErrorInvalidValue);
+  // across ranks A is the gathered buffer the plan was built on
+  if (pl->params.mode == kModeAgGemm && pl->params.world > 1 && A != pl->a_ptr) return static_cast<int>(cudaErrorInvalidValue);
+  CUtensorMap ta, tb;
+  const int e = encode_operands(pl, A, B, &ta, &tb);
+  return e != 0 ? e : run_plan(pl, ta, tb, epoch, stream);
 }
 
 int tcl_gemm_plan_set_operands(void* plan, const void* A, const void* B) {
   GemmPlan* pl = static_cast<GemmPlan*>(plan);
   if (!pl || !A || !B) return static_cast<int>(cudaErrorInvalidValue);
-  if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return static_cast<int>(cudaErrorMisalignedAddress);
   if (pl->params.mode == kModeAgGemm && A != pl->a_ptr) return static_cast<int>(cudaErrorInvalidValue);  // A is the gathered buffer the plan was built on
   CUtensorMap ta, tb;
-  if (ptx::encode_tmap_bf16_k64(&ta, A, static_cast<uint64_t>(pl->params.M), static_cast<uint64_t>(pl->params.K),
-                                static_cast<uint64_t>(pl->lda), 128) != 0 ||
-      ptx::encode_tmap_bf16_k64(&tb, B, static_cast<uint64_t>(pl->params.N), static_cast<uint64_t>(pl->params.K),
-                                static_cast<uint64_t>(pl->ldb), static_cast<uint32_t>(pl->params.b_box)) != 0)
-    return static_cast<int>(cudaErrorInvalidValue);
+  const int e = encode_operands(pl, A, B, &ta, &tb);
+  if (e != 0) return e;
   pl->tmap_a = ta;
   pl->tmap_b = tb;
   pl->a_ptr = A;

@@ -93,6 +93,9 @@ int tcl_gemm_plan_run(void* plan, int epoch, void* stream);
  * maps on the host; no device work).  Takes effect for launches made after it returns; not safe while another
  * thread launches the same plan.  For TCL_MODE_AG_GEMM, A is the gathered buffer and must stay what it was. */
 int tcl_gemm_plan_set_operands(void* plan, const void* A, const void* B);
+/* One launch on other operands of the plan's layout; the plan itself is not changed, so that several threads may do
+ * this at once.  With AG+GEMM across ranks A has to be the plan's gathered buffer; on one rank it may be any. */
+int tcl_gemm_plan_run_on(void* plan, const void* A, const void* B, int epoch, void* stream);
 void tcl_gemm_plan_destroy(void* plan);
 int tcl_gemm_plan_grid(void* plan);
 int tcl_gemm_smem_bytes(int cta_group);

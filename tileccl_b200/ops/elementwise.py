@@ -6,11 +6,10 @@ import ctypes as C
 import torch
 
 from .. import _native
+from ._plan import raw_stream
 
 
-def _stream_ptr(stream=None) -> C.c_void_p:
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return C.c_void_p(s.cuda_stream)
+_stream_ptr = raw_stream
 
 
 def silu_mul(gate_up: torch.Tensor, out: torch.Tensor | None = None, stream=None) -> torch.Tensor:
