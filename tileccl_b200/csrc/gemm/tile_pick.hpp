@@ -8,7 +8,8 @@
 //     the tensor work (546 cycles at 256 columns),
 //     the issue loop of the producer (240 cycles and 45 for each TMA load: 64 to 160 columns take the same time), or of
 //     the MMA warp, which comes to the same with two loads,
-//     its share of what the L2 delivers to all active CTAs (10000 bytes a cycle, 95 to one CTA);
+//     its share of what the L2 delivers to all active CTAs (10000 bytes a cycle, 95 to one CTA; half of that where K is not
+//     a multiple of 64: 1152 x 2816 x 1000 14.8 us one-CTA, 13.2 in pairs);
 //   128 columns of epilogue cost 1700 cycles; the epilogue of one tile overlaps the k-blocks of the next, the last
 //   one's is exposed; a CTA pair starts 2200 cycles later than a single CTA (cluster launch and barriers).
 // A narrower width has to gain more than kMargin: estimates closer than that came out either way from one board to the
@@ -40,7 +41,8 @@ inline double tile_cost(long long m, long long n, long long k, int cta_group, in
   const long long groups = ctas >= cta_group ? ctas / cta_group : 1;
   const long long waves = (tiles + groups - 1) / groups;
   const double active = static_cast<double>((tiles < groups ? tiles : groups) * cta_group);
-  const double bytes = 128.0 * 128.0 + 128.0 * bn / cta_group;      // per CTA and k-block
+  // per CTA and k-block; rows of 128 bytes that do not start on a 128-byte line touch two
+  const double bytes = (128.0 * 128.0 + 128.0 * bn / cta_group) * (k % 64 == 0 ? 1 : 2);
   double block = bn * (546.0 / 256.0);
   const double issue = 240.0 + 45.0 * (1 + bn / cta_group / b_box_rows(cta_group, bn, gate_up));
   if (block < issue) block = issue;

@@ -83,6 +83,13 @@ __device__ __forceinline__ bool wait_ge(const int* p, int target, volatile int* 
   }
 }
 
+// ---- programmatic dependent launch ------------------------------------------
+// Lets the next kernel of the stream start its CTAs (if it was launched for it) once every CTA here has said so or ended.
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Waits until the kernels before this one have completed and their memory operations are visible.  No-op in a kernel
+// that was launched the ordinary way.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- 128-bit data movers ----------------------------------------------------
 // Streaming load that does not allocate in L1 (peer memory is never cached in
 // the reader's L2, so L1 is the only cache that could return stale lines).
