@@ -63,6 +63,35 @@ def test_wide_gate_up_tiles(native_lib, num_ctas):
     assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("split,width", [(2, 64), (2, 192), (2, 256), (4, 128), (4, 256)])
+@pytest.mark.parametrize("M,N,K", [(128, 256, 256), (256, 768, 328), (128, 1792, 1000), (384, 512, 8192)])
+def test_split_k(native_lib, split, width, M, N, K):
+    from tileccl_b200.ops.gemm import GemmPlan
+    A, Bt = _operands(M, N, K)
+    out = torch.full((M + 1, N), 7.0, device="cuda", dtype=torch.bfloat16)
+    plan = GemmPlan(A, Bt, out=out[:M], cta_group=1, tile_cols=width, split_k=split, timeout_ms=1000)
+    assert native_lib.tcl_gemm_plan_split(plan.handle) == split
+    plan()
+    plan.check()
+    _same_as_reference(out[:M], A, Bt)
+    assert (out[M] == 7.0).all()
+    first = out.clone()
+    for _ in range(3):
+        plan()
+    plan.check()
+    assert torch.equal(out, first)
+
+
+def test_split_k_refuses_what_it_cannot_do(native_lib):
+    from tileccl_b200.ops.gemm import GemmPlan
+    A, Bt = _operands(512, 8192, 256)
+    for kw in (dict(cta_group=2, split_k=2), dict(cta_group=1, split_k=3), dict(cta_group=1, split_k=4, tile_cols=64),
+               dict(cta_group=1, split_k=2, tile_cols=128), dict(cta_group=1, split_k=2, tile_cols=256, num_ctas=64),
+               dict(cta_group=1, split_k=2, tile_cols=256, epi="silu_mul")):
+        with pytest.raises(ValueError):
+            GemmPlan(A, Bt, **kw)
+
+
 @pytest.mark.parametrize("M", [128, 384, 1152])
 @pytest.mark.parametrize("width", [32, 160, 256])
 def test_pair_with_a_half_empty_last_tile(native_lib, M, width):

@@ -71,6 +71,7 @@ class GemmDesc(C.Structure):
         ("epoch_dev", C.c_void_p),
         ("ragged_m", C.c_int32),
         ("tile_cols", C.c_int32),
+        ("split_k", C.c_int32),
     ]
 
 
@@ -124,6 +125,7 @@ def lib() -> C.CDLL:
     sig("tcl_gemm_pick_tile", i32, [i64, i64, i64, i32, i32, i32])
     sig("tcl_gemm_pick_form", i32, [i64, i64, i64, i32])
     sig("tcl_gemm_plan_tile_cols", i32, [vp])
+    sig("tcl_gemm_plan_split", i32, [vp])
     sig("tcl_sched_tile", None, [i32] * 8 + [C.POINTER(i32), C.POINTER(i32)])
     sig("tcl_barrier_all", i32, [C.POINTER(vp), i32, i32, i32, vp, u64, vp])
     sig("tcl_silu_mul", i32, [vp, vp, i64, i64, vp])

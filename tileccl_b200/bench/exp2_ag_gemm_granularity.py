@@ -85,7 +85,7 @@ class CePipeline:
             for c in range(seg // chunk_rows):
                 row0 = s * seg + c * chunk_rows
                 rows = a_full[row0:row0 + chunk_rows]
-                plan = GemmPlan(rows, Bt, out=out[row0:row0 + chunk_rows], cta_group=cta_group)
+                plan = GemmPlan(rows, Bt, out=out[row0:row0 + chunk_rows], cta_group=cta_group, split_k=1)
                 src = heap.peer_ptr(rows, s)
                 ev = torch.cuda.Event() if s != rank else None
                 self.chunks.append((s, src, rows.data_ptr(), rows.numel() * 2, ev, plan))
@@ -143,7 +143,7 @@ def main(argv=None) -> int:
         torch.distributed.all_gather_into_tensor(gathered, shard)
     else:
         gathered.copy_(shard)
-    full_plan = GemmPlan(gathered, Bt, out=out_ref, cta_group=args.cta_group)
+    full_plan = GemmPlan(gathered, Bt, out=out_ref, cta_group=args.cta_group, split_k=1)
     g2 = torch.empty(M, K, dtype=torch.bfloat16, device=dev)
     common = {"full": full_plan}
     if "nccl" in modes:

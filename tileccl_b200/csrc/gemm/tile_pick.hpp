@@ -35,12 +35,13 @@ inline int b_box_rows(int cta_group, int bn, bool gate_up) {
 }
 
 // Estimated SM cycles of an m x n x k GEMM in tiles of (128 * cta_group) x bn on `ctas` CTAs.
-inline double tile_cost(long long m, long long n, long long k, int cta_group, int ctas, int bn, bool gate_up) {
-  const long long kb = (k + 63) / 64;
+inline double tile_cost(long long m, long long n, long long k, int cta_group, int ctas, int bn, bool gate_up, int split = 1) {
+  const long long kb = ((k + 63) / 64 + split - 1) / split;
   const long long tiles = (m + 128 * cta_group - 1) / (128 * cta_group) * ((n + bn - 1) / bn);
-  const long long groups = ctas >= cta_group ? ctas / cta_group : 1;
+  const int per = cta_group * split;
+  const long long groups = ctas >= per ? ctas / per : 1;
   const long long waves = (tiles + groups - 1) / groups;
-  const double active = static_cast<double>((tiles < groups ? tiles : groups) * cta_group);
+  const double active = static_cast<double>((tiles < groups ? tiles : groups) * per);
   // per CTA and k-block; rows of 128 bytes that do not start on a 128-byte line touch two
   const double bytes = (128.0 * 128.0 + 128.0 * bn / cta_group) * (k % 64 == 0 ? 1 : 2);
   double block = bn * (546.0 / 256.0);
@@ -50,7 +51,8 @@ inline double tile_cost(long long m, long long n, long long k, int cta_group, in
   if (block < bytes * active / 10000.0) block = bytes * active / 10000.0;
   const double main_loop = static_cast<double>(kb) * block;
   const double epilogue = 1700.0 * ((bn + 127) / 128);
-  return static_cast<double>(waves) * (main_loop > epilogue ? main_loop : epilogue) + epilogue + (cta_group == 2 ? 2200.0 : 0.0);
+  return static_cast<double>(waves) * (main_loop > epilogue ? main_loop : epilogue) + epilogue + (per > 1 ? 2200.0 : 0.0) +
+         (split > 1 ? 1000.0 + (split - 1) * 512.0 * bn / split / 32.0 : 0.0);
 }
 
 // Columns per tile.
@@ -64,11 +66,35 @@ inline int pick_tile_cols(long long m, long long n, long long k, int cta_group, 
   return best;
 }
 
+// CTAs that share the k-blocks of a tile (one-CTA form), and that form's tile width with it: where the tiles do not fill
+// the chip, a cluster per tile reads fewer operand bytes than narrower tiles would.  What it pays is a cluster launch,
+// two cluster barriers and the exchange of (split - 1) / split of the fp32 accumulators (32 bytes a cycle).
+// Without and with, us: 128 x 8192 x 3584 14.0 -> 11.6 (2 CTAs, 128 columns), 128 x 3584 x 8192 26.2 -> 13.3 (4, 128), 512 x 1024 x
+// 8192 25.9 -> 13.5 (4, 128), 256 x 4096 x 4096 15.1 -> 12.4 (2, 128); not taken 256 x 4096 x 1024 6.8 against 7.9, 512 x 768 x 320 4.4 / 6.7.
+struct SplitPick { int split, cols; };
+inline SplitPick pick_split(long long m, long long n, long long k, int ctas, bool gate_up) {
+  SplitPick best{1, pick_tile_cols(m, n, k, 1, ctas, gate_up)};
+  if (gate_up) return best;
+  double cost = tile_cost(m, n, k, 1, ctas, best.cols, false) * (1.0 - kMargin);
+  for (int split = 2; split <= 4; split *= 2) {
+    // fours do not fill a GPC of the chip whose SMs are no multiple of four: leave some room
+    const long long room = split == 4 ? ctas - ctas / 8 : ctas;
+    for (int bn = kMaxTileCols; bn >= kTileColStep * split; bn -= kTileColStep * split) {
+      const long long tiles = (m + 127) / 128 * ((n + bn - 1) / bn);
+      if (tiles * split > room || (k + 63) / 64 < 4 * split) continue;
+      const double c = tile_cost(m, n, k, 1, ctas, bn, false, split);
+      if (c < cost) { cost = c; best = {split, bn}; }
+    }
+  }
+  return best;
+}
+
 // One CTA or a pair per tile, for rows that are a multiple of 128 (the pair's last tile may be half empty).  The pair
 // reads a third less from the L2; the single CTA starts earlier.  One-CTA against pair, us: 512 x 768 x 320 5.5 / 6.6,
 // 256 x 4096 x 4096 16.7 / 17.6, 512 x 8192 x 1024 11.2 / 12.2, 512 x 8192 x 3584 28.0 / 24.8, 4992 x 4096 x 4096 147 / 142.
 inline int pick_cta_group(long long m, long long n, long long k, int ctas) {
-  const double one = tile_cost(m, n, k, 1, ctas, pick_tile_cols(m, n, k, 1, ctas, false), false);
+  const SplitPick s = pick_split(m, n, k, ctas, false);
+  const double one = tile_cost(m, n, k, 1, ctas, s.cols, false, s.split);
   const double pair = tile_cost(m, n, k, 2, ctas, pick_tile_cols(m, n, k, 2, ctas, false), false);
   return one < pair ? 1 : 2;
 }

@@ -53,7 +53,7 @@ cudaError_t launch_gemm(const GemmPlan* pl, const CUtensorMap& tmap_a, const CUt
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = G;
+  attr[0].val.clusterDim.x = G * params.split;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
@@ -258,7 +258,7 @@ int tcl_gemm_desc_offset(const char* field) {
   TCL_OFF(mode) TCL_OFF(M) TCL_OFF(lda) TCL_OFF(A) TCL_OFF(world) TCL_OFF(seg_rows) TCL_OFF(dst_base) TCL_OFF(dst_row_off)
   TCL_OFF(rs_tile_cnt) TCL_OFF(rs_stage) TCL_OFF(rs_chunks) TCL_OFF(ag_src) TCL_OFF(ag_flags) TCL_OFF(gather_rows) TCL_OFF(ag_done)
   TCL_OFF(ag_push) TCL_OFF(ag_dst) TCL_OFF(barrier) TCL_OFF(status) TCL_OFF(timeout_ns) TCL_OFF(group_m) TCL_OFF(rs_mc_stage)
-  TCL_OFF(range_lo) TCL_OFF(epi_silu_mul) TCL_OFF(ablate) TCL_OFF(epi_st256) TCL_OFF(epi_tma_store) TCL_OFF(epoch_dev) TCL_OFF(ag_warps) TCL_OFF(ragged_m) TCL_OFF(tile_cols) TCL_OFF(rs_signal_batch) TCL_OFF(ag_vec32)
+  TCL_OFF(range_lo) TCL_OFF(epi_silu_mul) TCL_OFF(ablate) TCL_OFF(epi_st256) TCL_OFF(epi_tma_store) TCL_OFF(epoch_dev) TCL_OFF(ag_warps) TCL_OFF(ragged_m) TCL_OFF(tile_cols) TCL_OFF(split_k) TCL_OFF(rs_signal_batch) TCL_OFF(ag_vec32)
 #undef TCL_OFF
   return -1;
 }
@@ -271,6 +271,7 @@ int tcl_gemm_pick_tile(int64_t m, int64_t n, int64_t k, int cta_group, int ctas,
   return pick_cols(m, n, k, cta_group, ctas, gate_up != 0);
 }
 int tcl_gemm_pick_form(int64_t m, int64_t n, int64_t k, int ctas) { return pick_cta_group(m, n, k, ctas); }
+int tcl_gemm_plan_split(void* plan) { return plan ? static_cast<GemmPlan*>(plan)->params.split : 0; }
 int tcl_gemm_plan_tile_cols(void* plan) { return plan ? static_cast<GemmPlan*>(plan)->params.bn * static_cast<GemmPlan*>(plan)->params.halves : 0; }
 
 void tcl_sched_tile(int m_tiles, int n_tiles, int group_m, int order, int world, int rank,
@@ -381,12 +382,26 @@ void* tcl_gemm_plan_create(const tcl_gemm_desc* d, char* err, int errlen) {
   const bool local = d->world == 1 && !(d->mode == TCL_MODE_GEMM_RS && d->comm_enabled) && !d->epi_tma_store;
   const bool wide_ok = local && G == 2;
   int cols = local ? pick_cols(d->M, d->N, d->K, G, grid, d->epi_silu_mul != 0) : kMaxTileCols;
+  const bool split_ok = local && G == 1 && !d->epi_silu_mul && !d->epi_st256 && !d->ablate;
+  p.split = 1;
+  if (split_ok && d->split_k == 0 && d->tile_cols == 0) {
+    const SplitPick s = pick_split(d->M, d->N, d->K, grid, false);
+    p.split = s.split;
+    cols = s.cols;
+  }
   if (d->tile_cols) {
     const bool legal = d->tile_cols == 2 * kMaxTileCols ? wide_ok
                                                         : d->tile_cols >= kTileColStep && d->tile_cols <= kMaxTileCols && d->tile_cols % kTileColStep == 0;
     if (!legal || (!local && d->tile_cols != kMaxTileCols))
       return fail("tile_cols must be a multiple of 32 up to 256, or 512 in pairs, and 256 across ranks and with epi_tma_store");
     cols = d->tile_cols;
+  }
+  if (d->split_k) {
+    const long long tiles = static_cast<long long>(d->M / 128) * ((d->N + cols - 1) / cols);
+    if (d->split_k != 1 && (!split_ok || (d->split_k != 2 && d->split_k != 4) || cols % (kTileColStep * d->split_k) != 0 ||
+                            (d->K + 63) / 64 < d->split_k || tiles * d->split_k > grid))
+      return fail("split_k must be 1, 2 or 4, in the one-CTA form, with tile_cols a multiple of 32 * split_k and one tile per cluster");
+    p.split = d->split_k;
   }
   p.epi_warps = local && !d->epi_st256 && !d->ablate ? 8 : 4;
   p.halves = cols > kMaxTileCols ? 2 : 1;
@@ -485,7 +500,7 @@ void* tcl_gemm_plan_create(const tcl_gemm_desc* d, char* err, int errlen) {
       p.items += rest;
     }
   }
-  const int max_useful = p.items * G;
+  const int max_useful = p.items * G * p.split;
   if (grid > max_useful && (d->mode == TCL_MODE_PLAIN || local)) grid = max_useful;
   grid -= grid % G;
   if (grid < G) return fail("grid too small");

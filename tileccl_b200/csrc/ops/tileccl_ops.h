@@ -74,6 +74,7 @@ typedef struct tcl_gemm_desc {
   int32_t ragged_m;      /* cta_group 2, one row segment, no communication: M may be any multiple of 128 (the last pair's
                             second half lies below M; it is loaded as zeros and not stored) */
   int32_t tile_cols;     /* tile width in columns (a multiple of 32 up to 256, or 512 with cta_group 2), 0 = by estimate */
+  int32_t split_k;       /* cta_group 1, no communication: CTAs that share a tile's K, 1, 2 or 4; 0 = by estimate */
 } tcl_gemm_desc;
 
 /* Layout check for bindings that restate the struct: its size, and the offset of the named field
@@ -104,6 +105,7 @@ int tcl_gemm_smem_bytes(int cta_group);
 int tcl_gemm_pick_tile(int64_t m, int64_t n, int64_t k, int cta_group, int ctas, int gate_up);
 int tcl_gemm_pick_form(int64_t m, int64_t n, int64_t k, int ctas);
 int tcl_gemm_plan_tile_cols(void* plan);
+int tcl_gemm_plan_split(void* plan);
 /* Number of kernels one run launches (for launch accounting). */
 int tcl_gemm_plan_launches(void* plan);
 

@@ -171,6 +171,12 @@ __device__ __forceinline__ uint4 lds_v4(uint32_t addr) {
   return v;
 }
 
+// Store to another CTA's shared memory (a shared::cluster address from mapa).
+__device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(x), "r"(y), "r"(z), "r"(w)
+               : "memory");
+}
+
 // ---- NVLS multimem (addresses come from a multicast mapping of the heap) ------
 // Store 16 bytes to the same offset on every GPU bound to the multicast object.
 __device__ __forceinline__ void multimem_st_v4(void* mc_ptr, const uint4& v) {
