@@ -25,7 +25,6 @@ struct GemmPlan {
   OutMaps omaps;     // encoded only for the TMA-store epilogue
   int cta_group;
   int grid;
-  int early_launch;  // let the set-up of a launch overlap the kernel before it (programmatic dependent launch)
   int lda, ldb;      // operand row pitches (elements), kept for tcl_gemm_plan_set_operands
   const void* a_ptr;
 };
@@ -60,7 +59,7 @@ cudaError_t launch_gemm(const GemmPlan* pl, const CUtensorMap& tmap_a, const CUt
   cfg.numAttrs = 1;
   // Not across ranks: there CTAs wait for other CTAs and ranks, and an early CTA would hold an SM that they may need.
   // Back to back, launch latency, barrier and TMEM set-up of a call then hide behind the call before it.
-  if (pl->early_launch) {
+  if (params.early_dependents) {
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.numAttrs = 2;
@@ -506,7 +505,7 @@ void* tcl_gemm_plan_create(const tcl_gemm_desc* d, char* err, int errlen) {
   if (grid < G) return fail("grid too small");
   pl->grid = grid;
   pl->cta_group = G;
-  pl->early_launch = local && !d->ablate;
+  p.early_dependents = local && !d->ablate;
   pl->lda = d->lda;
   pl->ldb = d->ldb;
   pl->a_ptr = d->A;
