@@ -61,17 +61,18 @@ class Plan:
         return self.lib.tcl_gemm_plan_grid(self.handle)
 
     def run(self, stream: torch.cuda.Stream | None = None) -> None:
-        self._host_epoch += 1
-        rc = self.lib.tcl_gemm_plan_run(self.handle, self._host_epoch, raw_stream(stream))
-        _native.check(rc, "kernel launch")
-        self.launches += 1
+        self._launched(self.lib.tcl_gemm_plan_run(self.handle, self._host_epoch + 1, raw_stream(stream)))
 
     def run_on(self, A_ptr: int, B_ptr: int) -> None:
         """One launch on the current stream with operands at other addresses, of the layout the plan was built for
         (the caller has checked that): one call into the library that encodes two tensor maps and launches."""
-        self._host_epoch += 1
-        rc = self.lib.tcl_gemm_plan_run_on(self.handle, A_ptr, B_ptr, self._host_epoch, raw_stream())
+        self._launched(self.lib.tcl_gemm_plan_run_on(self.handle, A_ptr, B_ptr, self._host_epoch + 1, raw_stream()))
+
+    def _launched(self, rc: int) -> None:
+        # A call that was refused (a misaligned operand, say) is no call: its number goes to the next one, or this
+        # rank would wait for arrivals that its peers never make.
         _native.check(rc, "kernel launch")
+        self._host_epoch += 1
         self.launches += 1
 
     def set_operands(self, A: torch.Tensor, Bt: torch.Tensor) -> None:
