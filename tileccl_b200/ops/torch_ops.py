@@ -80,15 +80,16 @@ _lib.define("silu_mul(Tensor gate_up) -> Tensor")
 _lib.define("barrier() -> ()")
 
 
-def _form(m: int, n: int, k: int, world: int) -> dict:
+def _form(m: int, b_t: torch.Tensor, world: int) -> dict:
     """CTA form of a plan whose rank holds ``m`` rows.  One rank: whichever is estimated to be faster, the pair
-    also for an odd multiple of 128 rows (last tile half empty).  Several: the pair where its 256-row tiles fit."""
-    if _ctx["cta_group"] != 2 or m % 128:
+    also for an odd multiple of 128 rows (last tile half empty).  Several: the pair where its 256-row tiles fit.
+    Operands that no form takes are left to the plan, which says what is wrong with them."""
+    if _ctx["cta_group"] != 2 or m % 128 or b_t.dim() != 2:
         return {"cta_group": 1}
     if world > 1:
         return {"cta_group": 2 if m % 256 == 0 else 1}
     sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
-    if _native.lib().tcl_gemm_pick_form(m, n, k, sms) == 1:
+    if _native.lib().tcl_gemm_pick_form(m, *b_t.shape, sms) == 1:
         return {"cta_group": 1}
     return {"cta_group": 2, "ragged_m": m % 256 != 0}
 
@@ -97,7 +98,7 @@ def _gemm(a: torch.Tensor, b_t: torch.Tensor) -> torch.Tensor:
     k = _key("gemm", a, b_t)
     plan = _ctx["plans"].get(k)
     if plan is None:
-        plan = _ctx["plans"][k] = GemmPlan(a, b_t, hold_operands=False, **_form(a.shape[0], *b_t.shape, world=1))
+        plan = _ctx["plans"][k] = GemmPlan(a, b_t, hold_operands=False, **_form(a.shape[0], b_t, world=1))
         return plan()
     plan.run_on(a.data_ptr(), b_t.data_ptr())       # the key has checked everything but the addresses
     return plan.out
@@ -108,7 +109,7 @@ def _gemm_rs(a: torch.Tensor, b_t: torch.Tensor) -> torch.Tensor:
     op = _ctx["plans"].get(k)
     if op is None:
         h = heap()
-        op = _ctx["plans"][k] = GemmRs(h, a, b_t, hold_operands=False, **_form(a.shape[0] // h.world, *b_t.shape, world=h.world))
+        op = _ctx["plans"][k] = GemmRs(h, a, b_t, hold_operands=False, **_form(a.shape[0] // h.world, b_t, world=h.world))
         return op()
     op.plan.run_on(a.data_ptr(), b_t.data_ptr())
     return op.out
@@ -130,7 +131,7 @@ def _ag_gemm(a_shard: torch.Tensor, b_t: torch.Tensor, gather_rows: int = 512) -
     k = _key("ag_gemm", b_t, extra=(M, K, gather_rows))
     op = _ctx["plans"].get(k)
     if op is None:
-        op = _ctx["plans"][k] = AgGemm(h, M, K, b_t, gather_rows=gather_rows, hold_operands=False, **_form(a_shard.shape[0], *b_t.shape, world=h.world))
+        op = _ctx["plans"][k] = AgGemm(h, M, K, b_t, gather_rows=gather_rows, hold_operands=False, **_form(a_shard.shape[0], b_t, world=h.world))
     a_ptr = a_shard.data_ptr()
     if a_ptr != op.a_shard.data_ptr():
         if not _reads_in_place(h.world, a_shard, K, op.out):
