@@ -39,3 +39,38 @@ def test_chains_of_dependent_calls(native_lib, M):
             torch.cuda.synchronize()
             got = chain(lambda: None)
         assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("cta_group", [1, 2])
+def test_capped_calls_leave_the_other_sms_alone(native_lib, cta_group):
+    """Calls with a grid cap, back to back on one stream, hold no more SMs than the cap: a call on another stream that
+    fits in the rest runs beside the first of them, it does not wait for the last."""
+    from tileccl_b200.ops.gemm import GemmPlan
+    cap = torch.cuda.get_device_properties(0).multi_processor_count // 4 * 2 - 2
+    a, b = (torch.randn(4096, 8192, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    long = GemmPlan(a, b, cta_group=cta_group, num_ctas=cap, timeout_ms=1000)           # some 400 us a call
+    short = GemmPlan(a[:1024, :1024], b[:1024, :1024], cta_group=cta_group, num_ctas=cap, timeout_ms=1000)
+    streams = torch.cuda.Stream(), torch.cuda.Stream()
+    for s, plan in zip(streams, (long, short)):
+        s.wait_stream(torch.cuda.current_stream())
+        plan(s)                                                                          # loaded and warm
+    torch.cuda.synchronize()
+    begun, ended, beside = (torch.cuda.Event(enable_timing=True) for _ in range(3))
+    under_way = torch.cuda.Event()
+    calls = 10
+    with torch.cuda.stream(streams[0]):
+        begun.record()
+        long()
+        under_way.record()
+        for _ in range(calls - 1):
+            long()
+        ended.record()
+    with torch.cuda.stream(streams[1]):
+        streams[1].wait_event(under_way)
+        short()
+        beside.record()
+    torch.cuda.synchronize()
+    long.check()
+    short.check()
+    # beside the second call: over before that one is.  Behind calls that hold SMs ahead of their turn it ends with the third.
+    assert begun.elapsed_time(beside) < 2 * begun.elapsed_time(ended) / calls

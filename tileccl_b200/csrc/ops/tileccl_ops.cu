@@ -57,8 +57,7 @@ cudaError_t launch_gemm(const GemmPlan* pl, const CUtensorMap& tmap_a, const CUt
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  // Not across ranks: there CTAs wait for other CTAs and ranks, and an early CTA would hold an SM that they may need.
-  // Back to back, launch latency, barrier and TMEM set-up of a call then hide behind the call before it.
+  // Back to back, launch latency, barrier and TMEM set-up of a call then hide behind the end of the call before it.
   if (params.early_dependents) {
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
@@ -505,7 +504,10 @@ void* tcl_gemm_plan_create(const tcl_gemm_desc* d, char* err, int errlen) {
   if (grid < G) return fail("grid too small");
   pl->grid = grid;
   pl->cta_group = G;
-  p.early_dependents = local && !d->ablate;
+  // Not across ranks: there CTAs wait for other CTAs and ranks, and an early CTA would hold an SM that they may need.  Not
+  // with a grid cap either: its caller has given the other SMs away, and a call that waits beside the one before it
+  // would hold twice the cap.
+  p.early_dependents = local && !d->ablate && d->num_ctas <= 0;
   pl->lda = d->lda;
   pl->ldb = d->ldb;
   pl->a_ptr = d->A;

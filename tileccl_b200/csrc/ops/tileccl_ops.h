@@ -54,7 +54,7 @@ typedef struct tcl_gemm_desc {
   int32_t* status;      /* 4 ints, zeroed by the caller */
   uint64_t timeout_ns;  /* bound of every device-side wait; 0 = 4 s */
   int32_t group_m;      /* raster group height; 0 = default */
-  int32_t num_ctas;     /* 0 = one per SM */
+  int32_t num_ctas;     /* 0 = one per SM.  A cap also holds for what back-to-back launches occupy together */
   const void* rs_mc_stage; /* GEMM+RS NVLS variant: multicast mapping of the [M][N] staging buffer, else NULL */
   uint64_t range_lo[TCL_MAX_WORLD]; /* debug build: mapped range of the memory of rank s that this plan may touch */
   uint64_t range_hi[TCL_MAX_WORLD];
