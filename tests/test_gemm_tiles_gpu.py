@@ -130,3 +130,34 @@ def test_ops_take_odd_multiples_of_128_rows(native_lib, op, shape):
         tc.check_all()
     finally:
         tc.shutdown()
+
+
+@pytest.mark.parametrize("cta_group", [1, 2])
+def test_stores_of_the_epilogue_experiment_run_one_kernel_form(native_lib, cta_group):
+    """At a shape whose default one-CTA plan splits K: with comm_form every store has the same tiles and the same bits."""
+    from tileccl_b200.ops.gemm import GemmPlan
+    A, Bt = _operands(512, 1024, 8192)
+    if cta_group == 1:
+        assert native_lib.tcl_gemm_plan_split(GemmPlan(A, Bt, cta_group=1).handle) > 1
+    plans = [GemmPlan(A, Bt, cta_group=cta_group, store=s, comm_form=True, timeout_ms=1000) for s in ("st16", "st256", "tma")]
+    for p in plans:
+        assert (native_lib.tcl_gemm_plan_split(p.handle), native_lib.tcl_gemm_plan_tile_cols(p.handle)) == (1, 256)
+        p()
+        p.check()
+        assert torch.equal(p.out, plans[0].out)
+    _same_as_reference(plans[0].out, A, Bt)
+    with pytest.raises(ValueError):
+        GemmPlan(A, Bt, cta_group=cta_group, tile_cols=128, comm_form=True)
+    with pytest.raises(ValueError):
+        GemmPlan(A, Bt, cta_group=cta_group, split_k=2, comm_form=True)
+
+
+def test_epilogue_experiment_verifies_where_the_default_plan_splits_k():
+    import os
+    import subprocess
+    import sys
+    r = subprocess.run([sys.executable, "-m", "tileccl_b200.bench.exp3_epilogue_remote", "--cta-group", "1", "--epi", "st16,st256,tma", "--verify",
+                        "--sizes", "512x1024x8192", "--iters", "2", "--warmup", "1"],
+                       capture_output=True, text=True, timeout=300, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
+    assert r.stdout.count("| ok") == 2 and "FAIL" not in r.stdout, r.stdout

@@ -72,6 +72,7 @@ class GemmDesc(C.Structure):
         ("ragged_m", C.c_int32),
         ("tile_cols", C.c_int32),
         ("split_k", C.c_int32),
+        ("comm_form", C.c_int32),
     ]
 
 

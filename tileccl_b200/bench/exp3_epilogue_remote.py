@@ -75,7 +75,8 @@ def main(argv=None) -> int:
         nseg = M // seg
         plans = {}          # (mode, epilogue) -> plan
         for epi in epis:
-            kw = dict(out=D, cta_group=args.cta_group, store=epi)
+            # one kernel form for all of them: the rows differ by the store and its destination, and add the k-blocks in one order
+            kw = dict(out=D, cta_group=args.cta_group, store=epi, comm_form=True)
             for mode in modes:
                 if mode == "local":
                     plans[mode, epi] = GemmPlan(A, Bt, **kw)

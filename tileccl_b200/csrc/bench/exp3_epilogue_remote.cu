@@ -107,7 +107,7 @@ int main(int argc, char** argv) {
       tcl_gemm_desc d;
       std::memset(&d, 0, sizeof(d));
       d.mode = TCL_MODE_PLAIN; d.cta_group = cta_group; d.M = M; d.N = N; d.K = K; d.lda = K; d.ldb = K; d.ldc = N; d.A = A; d.B = B;
-      d.world = 1; d.status = status;
+      d.world = 1; d.status = status; d.comm_form = 1;
       if (m < 2) { d.seg_rows = M; d.dst_base[0] = m == 0 ? D.local : D.peer[peer]; }
       else {
         d.seg_rows = seg;

@@ -256,7 +256,7 @@ int tcl_gemm_desc_offset(const char* field) {
   TCL_OFF(mode) TCL_OFF(M) TCL_OFF(lda) TCL_OFF(A) TCL_OFF(world) TCL_OFF(seg_rows) TCL_OFF(dst_base) TCL_OFF(dst_row_off)
   TCL_OFF(rs_tile_cnt) TCL_OFF(rs_stage) TCL_OFF(rs_chunks) TCL_OFF(ag_src) TCL_OFF(ag_flags) TCL_OFF(gather_rows) TCL_OFF(ag_done)
   TCL_OFF(ag_push) TCL_OFF(ag_dst) TCL_OFF(barrier) TCL_OFF(status) TCL_OFF(timeout_ns) TCL_OFF(group_m) TCL_OFF(rs_mc_stage)
-  TCL_OFF(range_lo) TCL_OFF(epi_silu_mul) TCL_OFF(ablate) TCL_OFF(epi_st256) TCL_OFF(epi_tma_store) TCL_OFF(epoch_dev) TCL_OFF(ag_warps) TCL_OFF(ragged_m) TCL_OFF(tile_cols) TCL_OFF(split_k) TCL_OFF(rs_signal_batch) TCL_OFF(ag_vec32)
+  TCL_OFF(range_lo) TCL_OFF(epi_silu_mul) TCL_OFF(ablate) TCL_OFF(epi_st256) TCL_OFF(epi_tma_store) TCL_OFF(epoch_dev) TCL_OFF(ag_warps) TCL_OFF(ragged_m) TCL_OFF(tile_cols) TCL_OFF(split_k) TCL_OFF(comm_form) TCL_OFF(rs_signal_batch) TCL_OFF(ag_vec32)
 #undef TCL_OFF
   return -1;
 }
@@ -376,8 +376,9 @@ void* tcl_gemm_plan_create(const tcl_gemm_desc* d, char* err, int errlen) {
   if (grid > sms) grid = sms;
 
   // The width is free where a tile is nobody else's unit: not across ranks (counters and reduce warps take 128 x 256
-  // tiles), not with the TMA-store epilogue (its boxes are 64 columns wide and would run over the next tile).
-  const bool local = d->world == 1 && !(d->mode == TCL_MODE_GEMM_RS && d->comm_enabled) && !d->epi_tma_store;
+  // tiles), not with the TMA-store epilogue (its boxes are 64 columns wide and would run over the next tile), not where the
+  // caller wants the form of those plans.
+  const bool local = !d->comm_form && d->world == 1 && !(d->mode == TCL_MODE_GEMM_RS && d->comm_enabled) && !d->epi_tma_store;
   const bool wide_ok = local && G == 2;
   int cols = local ? pick_cols(d->M, d->N, d->K, G, grid, d->epi_silu_mul != 0) : kMaxTileCols;
   const bool split_ok = local && G == 1 && !d->epi_silu_mul && !d->epi_st256 && !d->ablate;
@@ -391,7 +392,7 @@ void* tcl_gemm_plan_create(const tcl_gemm_desc* d, char* err, int errlen) {
     const bool legal = d->tile_cols == 2 * kMaxTileCols ? wide_ok
                                                         : d->tile_cols >= kTileColStep && d->tile_cols <= kMaxTileCols && d->tile_cols % kTileColStep == 0;
     if (!legal || (!local && d->tile_cols != kMaxTileCols))
-      return fail("tile_cols must be a multiple of 32 up to 256, or 512 in pairs, and 256 across ranks and with epi_tma_store");
+      return fail("tile_cols must be a multiple of 32 up to 256, or 512 in pairs, and 256 across ranks, with epi_tma_store and with comm_form");
     cols = d->tile_cols;
   }
   if (d->split_k) {

@@ -75,6 +75,8 @@ typedef struct tcl_gemm_desc {
                             second half lies below M; it is loaded as zeros and not stored) */
   int32_t tile_cols;     /* tile width in columns (a multiple of 32 up to 256, or 512 with cta_group 2), 0 = by estimate */
   int32_t split_k;       /* cta_group 1, no communication: CTAs that share a tile's K, 1, 2 or 4; 0 = by estimate */
+  int32_t comm_form;     /* take the kernel form that communicating plans have, also where nothing is communicated: 256-column
+                            tiles, unsplit K, four epilogue warps that store 256 bytes of a row together, ordinary launch */
 } tcl_gemm_desc;
 
 /* Layout check for bindings that restate the struct: its size, and the offset of the named field
