@@ -152,12 +152,16 @@ def test_stores_of_the_epilogue_experiment_run_one_kernel_form(native_lib, cta_g
         GemmPlan(A, Bt, cta_group=cta_group, split_k=2, comm_form=True)
 
 
-def test_epilogue_experiment_verifies_where_the_default_plan_splits_k():
+@pytest.mark.parametrize("args,checks", [
+    ("exp3_epilogue_remote --cta-group 1 --epi st16,st256,tma --sizes 512x1024x8192", 2),
+    ("exp2_ag_gemm_granularity --cta-group 1 --m 512 --n 1024 --k 8192 --modes fused,ce --gather-rows 256,512", 4),
+])
+def test_experiments_verify_where_the_default_plan_splits_k(args, checks):
     import os
     import subprocess
     import sys
-    r = subprocess.run([sys.executable, "-m", "tileccl_b200.bench.exp3_epilogue_remote", "--cta-group", "1", "--epi", "st16,st256,tma", "--verify",
-                        "--sizes", "512x1024x8192", "--iters", "2", "--warmup", "1"],
+    module, *flags = args.split()
+    r = subprocess.run([sys.executable, "-m", f"tileccl_b200.bench.{module}", *flags, "--verify", "--iters", "2", "--warmup", "1"],
                        capture_output=True, text=True, timeout=300, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
-    assert r.stdout.count("| ok") == 2 and "FAIL" not in r.stdout, r.stdout
+    assert r.stdout.count("| ok") == checks and "FAIL" not in r.stdout, r.stdout

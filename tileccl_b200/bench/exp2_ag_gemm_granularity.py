@@ -85,7 +85,7 @@ class CePipeline:
             for c in range(seg // chunk_rows):
                 row0 = s * seg + c * chunk_rows
                 rows = a_full[row0:row0 + chunk_rows]
-                plan = GemmPlan(rows, Bt, out=out[row0:row0 + chunk_rows], cta_group=cta_group, split_k=1)
+                plan = GemmPlan(rows, Bt, out=out[row0:row0 + chunk_rows], cta_group=cta_group, comm_form=True)
                 src = heap.peer_ptr(rows, s)
                 ev = torch.cuda.Event() if s != rank else None
                 self.chunks.append((s, src, rows.data_ptr(), rows.numel() * 2, ev, plan))
@@ -143,7 +143,9 @@ def main(argv=None) -> int:
         torch.distributed.all_gather_into_tensor(gathered, shard)
     else:
         gathered.copy_(shard)
-    full_plan = GemmPlan(gathered, Bt, out=out_ref, cta_group=args.cta_group, split_k=1)
+    # comm_form everywhere: all variants run the kernel form that the fused one has across ranks, so that the times differ by the
+    # transfers alone and the bits not at all
+    full_plan = GemmPlan(gathered, Bt, out=out_ref, cta_group=args.cta_group, comm_form=True)
     g2 = torch.empty(M, K, dtype=torch.bfloat16, device=dev)
     common = {"full": full_plan}
     if "nccl" in modes:
@@ -157,13 +159,13 @@ def main(argv=None) -> int:
         S = seg // g
         for mode in [m for m in modes if m in ("fused", "ce")]:
             if mode == "fused":
-                op = AgGemm(heap, M, K, Bt, cta_group=args.cta_group, gather_rows=g, out=out, ablate=args.ablate, transport=args.transport, item_rows=args.item_rows)
+                op = AgGemm(heap, M, K, Bt, cta_group=args.cta_group, gather_rows=g, out=out, ablate=args.ablate, transport=args.transport, item_rows=args.item_rows, comm_form=True)
                 ctrl = None
                 a_full = op.a_full
                 op.a_shard.copy_(shard)
                 run_ovl = lambda: op()
                 # t_seg: same kernel, same tile order, no waiting (data already gathered)
-                seg_op = AgGemm(heap, M, K, Bt, cta_group=args.cta_group, gather_rows=g, out=out, comm_enabled=False, transport=args.transport)
+                seg_op = AgGemm(heap, M, K, Bt, cta_group=args.cta_group, gather_rows=g, out=out, comm_enabled=False, transport=args.transport, comm_form=True)
                 seg_op.a_full.copy_(gathered)
                 run_seg = lambda: seg_op()
                 run_comm = None

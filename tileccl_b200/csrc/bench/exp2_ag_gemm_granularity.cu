@@ -147,7 +147,7 @@ int main(int argc, char** argv) {
     std::memset(&d, 0, sizeof(d));
     d.mode = TCL_MODE_PLAIN; d.cta_group = cta_group; d.M = M; d.N = N; d.K = K; d.lda = K; d.ldb = K; d.ldc = N; d.A = gathered; d.B = B;
     d.world = 1; d.seg_rows = M; d.dst_base[0] = out_ref; d.status = status;
-    d.split_k = 1;      // compared bit for bit with the fused kernel, which adds the k-blocks in order
+    d.comm_form = 1;    // compared with the fused kernel, in time and bit for bit: the same tiles, the k-blocks added in order
     void* p = tcl_gemm_plan_create(&d, err, sizeof(err));
     if (!p) die(L, err);
     return p;
@@ -164,7 +164,7 @@ int main(int argc, char** argv) {
       d.barrier[s] = static_cast<int32_t*>(bar_k.peer[s]);
     }
     d.ag_flags = static_cast<int32_t*>(flags.local); d.gather_rows = gather_rows; d.ag_item_rows = 1; d.ag_done = static_cast<int32_t*>(done.local);
-    d.status = status;
+    d.status = status; d.comm_form = 1;
     void* p = tcl_gemm_plan_create(&d, err, sizeof(err));
     if (!p) die(L, err);
     return p;
@@ -186,7 +186,7 @@ int main(int argc, char** argv) {
     d.mode = TCL_MODE_PLAIN; d.cta_group = (rows % (128 * cta_group) == 0) ? cta_group : 1; d.M = rows; d.N = N; d.K = K; d.lda = K; d.ldb = K; d.ldc = N;
     d.A = static_cast<char*>(afull.local) + row0 * K * 2; d.B = B;
     d.world = 1; d.seg_rows = rows; d.dst_base[0] = static_cast<char*>(out) + row0 * N * 2; d.status = status;
-    d.split_k = 1;
+    d.comm_form = 1;
     void* p = tcl_gemm_plan_create(&d, err, sizeof(err));
     if (!p) die(L, err);
     return p;

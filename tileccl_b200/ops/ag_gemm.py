@@ -39,7 +39,7 @@ class AgGemm:
     def __init__(self, heap: SymmetricHeap, M: int, K: int, Bt: torch.Tensor, cta_group: int = 2,
                  gather_rows: int = 512, out: torch.Tensor | None = None, group_m: int = 0,
                  num_ctas: int = 0, comm_enabled: bool = True, timeout_ms: float = 4000.0, ablate: int = 0, transport: str = "pull", item_rows: int = 1, epi: str | None = None,
-                 device_epoch: bool = False, hold_operands: bool = True, gather_warps: int = 0, vec32: bool = False, ragged_m: bool = False):
+                 device_epoch: bool = False, hold_operands: bool = True, gather_warps: int = 0, vec32: bool = False, ragged_m: bool = False, comm_form: bool = False):
         require_bf16_rowmajor(Bt, "Bt")
         self.heap = heap
         world, rank = heap.world, heap.rank
@@ -101,6 +101,7 @@ class AgGemm:
         d.group_m, d.num_ctas = group_m, num_ctas
         d.ablate = ablate
         d.ragged_m = 1 if ragged_m else 0
+        d.comm_form = 1 if comm_form else 0      # on one rank: the kernel form that several ranks have, see GemmPlan
         own = (out, self.a_full, self.flags, self.done, self.barrier)
         self.plan = Plan(d, keep_alive=((Bt,) + own) if hold_operands else own, device_epoch=device_epoch)
         self.gather_rows = gather_rows
