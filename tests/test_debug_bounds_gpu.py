@@ -52,3 +52,43 @@ def test_debug_build_checks_addresses():
     r = subprocess.run([sys.executable, "-c", CODE], capture_output=True, text=True, timeout=300, env=env, cwd=root)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-3000:]
     assert "GOOD_RUN_OK" in r.stdout and "STATUS 9" in r.stdout and "BAD_RANGE_REFUSED" in r.stdout
+
+
+DIRECT = r"""
+import ctypes as C
+import torch
+from tileccl_b200 import _build, _native
+_build.build(programs=False)
+from tileccl_b200.ops.gemm_rs import GemmRs
+from tileccl_b200.ops._plan import KernelTimeout
+from tileccl_b200.parallel.heap import SymmetricHeap
+heap = SymmetricHeap(64 << 20)
+# on one rank the epilogue writes the result itself: eight-warp stores (pair, one CTA), and the stores of a split K
+for cta_group, K, split in ((2, 256, 1), (1, 256, 1), (1, 8192, 4)):
+    A = torch.randn(512, K, device="cuda", dtype=torch.bfloat16)
+    Bt = torch.randn(1024, K, device="cuda", dtype=torch.bfloat16)
+    op = GemmRs(heap, A, Bt, cta_group=cta_group, timeout_ms=300)
+    op(); op.check()
+    lib, d = op.plan.lib, op.plan.desc
+    lib.tcl_gemm_plan_destroy(op.plan.handle)
+    d.range_hi[0] = d.range_lo[0] + 16
+    err = C.create_string_buffer(256)
+    op.plan.handle = lib.tcl_gemm_plan_create(C.byref(d), err, 256)
+    assert lib.tcl_gemm_plan_split(op.plan.handle) == split
+    op.out.fill_(7.0)
+    op()
+    try:
+        op.check()
+        raise SystemExit("a store outside the range went unnoticed")
+    except KernelTimeout as e:
+        assert e.code == 9, e
+    assert (op.out == 7.0).all()
+print("DIRECT_STORES_REFUSED")
+"""
+
+
+def test_debug_build_checks_the_stores_of_a_single_rank():
+    env = dict(os.environ, TILECCL_DEBUG="1")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", DIRECT], capture_output=True, text=True, timeout=300, env=env, cwd=root)
+    assert r.returncode == 0 and "DIRECT_STORES_REFUSED" in r.stdout, r.stdout[-2000:] + r.stderr[-3000:]
