@@ -35,5 +35,42 @@ def test_silu_mul_every_gate_value(native_lib):
     assert (out[gate == float("inf")] == float("inf")).all()
     ref = gate.double() * torch.sigmoid(gate.double())
     err = (out.double() - ref).abs()
-    # exp(-|g|) carries up to 2 + 1.2 |g| fp32 steps (its documented bound), which stays inside a bf16 half step up to |g| = 100
+    # exp(-|g|) carries up to 2 + 1.2 |g| fp32 steps (its documented bound): far inside a bf16 half step.  From -87.4 down it is
+    # subnormal and less precise, but these results are below 4e-36 times up = 1; a large up shows them, in the next test
     assert (err[finite] <= (ref.abs() * (2.0 ** -8 + 2.0 ** -16) + 2e-37)[finite]).all()
+
+
+def test_silu_mul_gates_whose_exponential_is_subnormal(native_lib):
+    from tileccl_b200.ops import elementwise as ew
+    gate = torch.arange(-104, -80, 0.5, device="cuda").bfloat16().repeat(8, 2)[:, :96].contiguous()
+    up = torch.full_like(gate, 1e36)
+    out = ew.silu_mul(torch.cat([gate, up], 1).contiguous())
+    g, u = gate.double(), up.double()
+    ref = g * torch.sigmoid(g) * u
+    # exp(-|g|) to its documented 2 + 1.173 |g| fp32 steps or to one subnormal quantum, its product with the gate to half a
+    # quantum, and half a bf16 step
+    tol = ref.abs() * (2.0 ** -8 * 1.01 + 130 * 2.0 ** -23) + (g.abs() + 0.5) * 2.0 ** -149 * u
+    assert ((out.double() - ref).abs() <= tol).all()
+    assert (out[gate > -100] != 0).all()
+
+
+def test_silu_mul_rounds_like_a_correctly_rounded_divide(native_lib):
+    """fp32 errors show in bf16 results where the exact value lies next to a midpoint.  A chain with a correctly rounded
+    divide picks the wrong neighbour for 56 of these results, one with a divide of two fp32 steps for 228."""
+    from tileccl_b200.ops import elementwise as ew
+    gen = torch.Generator(device="cuda").manual_seed(0)
+    gu = torch.empty(16384, 2 * 3584, device="cuda", dtype=torch.bfloat16).normal_(generator=gen)
+    out = ew.silu_mul(gu)
+    wrong = 0
+    for rows in range(0, gu.shape[0], 2048):
+        g, u = gu[rows:rows + 2048].double().split(3584, dim=1)
+        wrong += int((out[rows:rows + 2048] != (g * torch.sigmoid(g) * u).bfloat16()).sum())
+    assert wrong <= 100
+
+
+def test_silu_mul_keeps_the_sign_of_zero(native_lib):
+    from tileccl_b200.ops import elementwise as ew
+    gate = torch.tensor([0.0, -0.0, -200.0, 0.0] * 4, device="cuda").bfloat16()
+    up = torch.tensor([1.0, 1.0, 1.0, -1.0] * 4, device="cuda").bfloat16()
+    out = ew.silu_mul(torch.cat([gate, up])[None])
+    assert torch.equal(torch.signbit(out)[0], torch.tensor([False, True, True, True] * 4, device="cuda")) and (out == 0).all()

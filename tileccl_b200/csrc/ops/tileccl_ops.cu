@@ -117,8 +117,8 @@ __global__ void barrier_all_kernel(BarrierArgs a, int world, int rank, int epoch
 // elements, a block's width apart, all loads issued before the first use; one block per slice of the output
 // instead of a grid-stride loop, so that the tail is one block deep.  What it must not be bound by is the
 // instruction issue: with an IEEE divide per element, a 64-bit divide per chunk and 16-byte loads in a grid-stride
-// loop 16384 x 3584 took 69.8 us (5.05 TB/s), now 54.4 us (6.48 TB/s); 32768 x 1000 43.0 -> 29.1 us, 1000 x 14336
-// 20.9 -> 14.7 us.  See silu_mul_f32, and the row of a chunk is found in 32 bits where the count allows it.
+// loop 16384 x 3584 took 69.8 us (5.05 TB/s), now 54.6 us (6.46 TB/s); in 16-byte chunks 32768 x 1000 43.0 -> 32.8 us
+// and 4096 x 4104 24.6 -> 18.4 us.  See silu_mul_f32, and the row of a chunk is found in 32 bits where the count allows it.
 // ---------------------------------------------------------------------------
 struct Vec4 {
   uint32_t w[4];
