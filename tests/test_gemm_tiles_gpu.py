@@ -165,3 +165,28 @@ def test_experiments_verify_where_the_default_plan_splits_k(args, checks):
                        capture_output=True, text=True, timeout=300, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
     assert r.stdout.count("| ok") == checks and "FAIL" not in r.stdout, r.stdout
+
+
+@pytest.mark.parametrize("cta_group", [1, 2])
+def test_base_ctrl_and_fused_of_the_reduce_scatter_experiment_run_the_same_tiles(native_lib, cta_group):
+    """Also on one rank, at a shape where a plan left to itself takes other tiles (one CTA: K split, pair: narrower)."""
+    from tileccl_b200.ops.gemm import GemmPlan
+    from tileccl_b200.ops.gemm_rs import GemmRs
+    from tileccl_b200.parallel.heap import SymmetricHeap
+    A, Bt = _operands(512, 1024, 8192)
+
+    def form(handle):
+        return native_lib.tcl_gemm_plan_split(handle), native_lib.tcl_gemm_plan_tile_cols(handle)
+
+    assert form(GemmPlan(A, Bt, cta_group=cta_group).handle) != (1, 256)
+    heap = SymmetricHeap(128 << 20)
+    try:
+        ops = [GemmRs(heap, A, Bt, cta_group=cta_group, comm_form=True, timeout_ms=1000, **kw) for kw in ({}, {"comm_enabled": False}, {"force_staged": True})]
+        base = GemmPlan(A, Bt, cta_group=cta_group, comm_form=True, timeout_ms=1000)
+        assert {form(base.handle), *(form(op.plan.handle) for op in ops)} == {(1, 256)}
+        want = base()
+        for op in (ops[0], ops[2]):          # ctrl leaves its result in the staging buffer
+            assert torch.equal(op(), want)
+            op.check()
+    finally:
+        heap.close()

@@ -83,11 +83,12 @@ def main(argv=None) -> int:
         ew.fill_normal_(A, seed=1000 + rank)
         ew.fill_normal_(Bt, seed=2000 + rank)
         D = torch.empty(M, N, dtype=torch.bfloat16, device=dev)
-        plain = GemmPlan(A, Bt, out=D, cta_group=args.cta_group)
+        # comm_form: base, ctrl and fused run the same tiles, so that their differences are the roles and the communication
+        plain = GemmPlan(A, Bt, out=D, cta_group=args.cta_group, comm_form=True)
         fused = GemmRs(heap, A, Bt, cta_group=args.cta_group, rs_chunks=args.rs_chunks, group_m=args.group_m, num_ctas=args.num_ctas,
-                       ablate=args.ablate, transport=args.transport, st256=args.st256)
+                       ablate=args.ablate, transport=args.transport, st256=args.st256, comm_form=True)
         ctrl = GemmRs(heap, A, Bt, cta_group=args.cta_group, rs_chunks=args.rs_chunks, group_m=args.group_m, num_ctas=args.num_ctas,
-                      comm_enabled=False)
+                      comm_enabled=False, comm_form=True)
         bar = ew.DeviceBarrier(heap)
         out_nccl = torch.empty(M // world, N, dtype=torch.bfloat16, device=dev) if world > 1 else None
         flush = None if args.no_flush else L2Flusher()

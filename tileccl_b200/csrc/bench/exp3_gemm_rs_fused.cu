@@ -147,7 +147,7 @@ int main(int argc, char** argv) {
     tcl_gemm_desc d;
     std::memset(&d, 0, sizeof(d));
     d.mode = mode; d.cta_group = cta_group; d.M = M; d.N = N; d.K = K; d.lda = K; d.ldb = K; d.ldc = N; d.A = A; d.B = B;
-    d.status = status;
+    d.status = status; d.comm_form = 1;   // base, ctrl and fused on the same tiles
     if (mode == TCL_MODE_PLAIN) { d.world = 1; d.rank = 0; d.seg_rows = M; d.dst_base[0] = D; }
     else {
       d.world = world; d.rank = rank; d.seg_rows = seg; d.comm_enabled = comm;
