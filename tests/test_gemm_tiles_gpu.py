@@ -190,3 +190,39 @@ def test_base_ctrl_and_fused_of_the_reduce_scatter_experiment_run_the_same_tiles
             op.check()
     finally:
         heap.close()
+
+
+@pytest.mark.parametrize("cta_group,K", [(1, 8192), (2, 512)])
+def test_routed_outputs_take_the_form_measured_at_peers(native_lib, cta_group, K):
+    from tileccl_b200.ops.gemm import GemmPlan
+    A, Bt = _operands(512, 1024, K)
+    parts = [torch.full((128 * cta_group, 1024), 7.0, device="cuda", dtype=torch.bfloat16) for _ in range(4 // cta_group)]
+    plan = GemmPlan(A, Bt, cta_group=cta_group, seg_rows=128 * cta_group, dst_ptrs=[t.data_ptr() for t in parts], timeout_ms=1000)
+    assert (native_lib.tcl_gemm_plan_split(plan.handle), native_lib.tcl_gemm_plan_tile_cols(plan.handle)) == (1, 256)
+    plan()
+    plan.check()
+    _same_as_reference(torch.cat(parts), A, Bt)
+
+
+@pytest.mark.parametrize("kw", [dict(cta_group=1, tile_cols=96), dict(cta_group=1, tile_cols=128, split_k=2), dict(cta_group=1, tile_cols=256, split_k=4),
+                                dict(cta_group=2, tile_cols=160), dict(cta_group=2, tile_cols=512), dict(cta_group=2, tile_cols=512, num_ctas=6)])
+@pytest.mark.parametrize("segments", [2, 4])
+def test_row_segments_on_every_form(native_lib, kw, segments):
+    """Segments routed to separate buffers in shuffled order, on the forms that find segment and row offset by themselves."""
+    from tileccl_b200.ops.gemm import GemmPlan
+    M, N = 1024, 768
+    A, Bt = _operands(M, N, 1000)
+    rows = M // segments
+    parts = [torch.full((rows + 1, N), 7.0, device="cuda", dtype=torch.bfloat16) for _ in range(segments)]
+    order = list(range(1, segments)) + [0]
+    plan = GemmPlan(A, Bt, seg_rows=rows, dst_ptrs=[parts[i].data_ptr() for i in order], comm_form=False, timeout_ms=1000, **kw)
+    plan()
+    plan.check()
+    _same_as_reference(torch.cat([parts[i][:rows] for i in order]), A, Bt)
+    assert all((t[rows] == 7.0).all() for t in parts)
+    # and through the row offsets of one output
+    out = torch.full((M + 1, N), 7.0, device="cuda", dtype=torch.bfloat16)
+    plan = GemmPlan(A, Bt, out=out[:M], seg_rows=rows, timeout_ms=1000, **kw)
+    plan()
+    plan.check()
+    assert torch.equal(out[:M], torch.cat([parts[i][:rows] for i in order])) and (out[M] == 7.0).all()

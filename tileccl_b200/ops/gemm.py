@@ -16,7 +16,7 @@ class GemmPlan(Plan):
     def __init__(self, A: torch.Tensor, Bt: torch.Tensor, out: torch.Tensor | None = None,
                  cta_group: int = 2, group_m: int = 0, num_ctas: int = 0, timeout_ms: float = 4000.0,
                  dst_ptrs: list[int] | None = None, seg_rows: int | None = None, epi: str | None = None,
-                 store: str = "st16", hold_operands: bool = True, ragged_m: bool = False, tile_cols: int = 0, split_k: int = 0, comm_form: bool = False):
+                 store: str = "st16", hold_operands: bool = True, ragged_m: bool = False, tile_cols: int = 0, split_k: int = 0, comm_form: bool | None = None):
         """``dst_ptrs``/``seg_rows`` route row segments of D to other addresses
         (a peer's buffer): the epilogue-remote experiment.  ``store`` picks how the epilogue leaves the
         SM: ``st16`` (16-byte st.global, the default), ``st256`` (32-byte st.global.v8.b32) or ``tma``
@@ -26,7 +26,9 @@ class GemmPlan(Plan):
         ``tile_cols`` fixes the width of a tile (a multiple of 32 up to 256, or 512 in pairs; 0 = chosen for the shape) and
         ``split_k`` the CTAs that share a tile's K in the one-CTA form (1, 2 or 4; 0 = chosen); ``comm_form`` takes the
         kernel form of the communicating plans (256-column tiles, unsplit K, four epilogue warps, ordinary launch): what a
-        comparison with them, or of one ``store`` with another, has to run on both sides."""
+        comparison with them, or of one ``store`` with another, has to run on both sides.  It is the default with
+        ``dst_ptrs``, which may be peers' memory: only its stores (256 contiguous bytes per row) were measured over NVLink,
+        the others write 128 bytes of a row together, and 16 where K is split."""
         if store not in ("st16", "st256", "tma"):
             raise ValueError("store must be st16, st256 or tma")
         require_bf16_rowmajor(A, "A")
@@ -63,7 +65,7 @@ class GemmPlan(Plan):
         d.ragged_m = 1 if ragged_m else 0
         d.tile_cols = tile_cols
         d.split_k = split_k
-        d.comm_form = 1 if comm_form else 0
+        d.comm_form = 1 if (bool(dst_ptrs) if comm_form is None else comm_form) else 0
         # hold_operands=False: the caller re-points the plan with set_operands() and owns the operands' lifetime
         super().__init__(d, keep_alive=(A, Bt, out) if hold_operands else (out,))
         self.out = out
