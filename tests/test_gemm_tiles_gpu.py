@@ -82,6 +82,24 @@ def test_split_k(native_lib, split, width, M, N, K):
     assert torch.equal(out, first)
 
 
+@pytest.mark.parametrize("M", [128, 512])
+@pytest.mark.parametrize("N", [256, 1024, 2048])
+def test_split_k_alone_finds_its_width(native_lib, M, N):
+    """split_k without tile_cols: refused only where no width fits; and a plan has the width and split that the rule names."""
+    from tileccl_b200.ops.gemm import GemmPlan
+    A, Bt = _operands(M, N, 4096)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for split in (2, 4):
+        assert M // 128 * -(-N // 256) * split <= sms
+        plan = GemmPlan(A, Bt, cta_group=1, split_k=split, timeout_ms=1000)
+        assert native_lib.tcl_gemm_plan_split(plan.handle) == split
+        _same_as_reference(plan(), A, Bt)
+        plan.check()
+    plan = GemmPlan(A, Bt, cta_group=1)
+    assert native_lib.tcl_gemm_plan_tile_cols(plan.handle) == native_lib.tcl_gemm_pick_tile(M, N, 4096, 1, sms, 0)
+    assert native_lib.tcl_gemm_plan_split(plan.handle) == native_lib.tcl_gemm_pick_split(M, N, 4096, sms)
+
+
 def test_split_k_refuses_what_it_cannot_do(native_lib):
     from tileccl_b200.ops.gemm import GemmPlan
     A, Bt = _operands(512, 8192, 256)

@@ -125,6 +125,7 @@ def lib() -> C.CDLL:
     sig("tcl_gemm_smem_bytes", i32, [i32])
     sig("tcl_gemm_pick_tile", i32, [i64, i64, i64, i32, i32, i32])
     sig("tcl_gemm_pick_form", i32, [i64, i64, i64, i32])
+    sig("tcl_gemm_pick_split", i32, [i64, i64, i64, i32])
     sig("tcl_gemm_plan_tile_cols", i32, [vp])
     sig("tcl_gemm_plan_split", i32, [vp])
     sig("tcl_sched_tile", None, [i32] * 8 + [C.POINTER(i32), C.POINTER(i32)])

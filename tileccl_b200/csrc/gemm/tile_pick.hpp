@@ -72,19 +72,31 @@ inline int pick_tile_cols(long long m, long long n, long long k, int cta_group, 
 // Without and with, us: 128 x 8192 x 3584 14.0 -> 11.6 (2 CTAs, 128 columns), 128 x 3584 x 8192 26.2 -> 13.3 (4, 128), 512 x 1024 x
 // 8192 25.9 -> 13.5 (4, 128), 256 x 4096 x 4096 15.1 -> 12.4 (2, 128); not taken 256 x 4096 x 1024 6.8 against 7.9, 512 x 768 x 320 4.4 / 6.7.
 struct SplitPick { int split, cols; };
+
+// The width for a given split (2 or 4) and its estimate; no width (0) where the tiles do not fit the chip side by side or a
+// CTA would get no k-block.
+inline int pick_split_cols(long long m, long long n, long long k, int ctas, int split, double* cost) {
+  int best = 0;
+  for (int bn = kMaxTileCols; bn >= kTileColStep * split; bn -= kTileColStep * split) {
+    const long long tiles = (m + 127) / 128 * ((n + bn - 1) / bn);
+    if (tiles * split > ctas || (k + 63) / 64 < split) continue;
+    const double c = tile_cost(m, n, k, 1, ctas, bn, false, split);
+    if (best == 0 || c < *cost) { best = bn; *cost = c; }
+  }
+  return best;
+}
+
 inline SplitPick pick_split(long long m, long long n, long long k, int ctas, bool gate_up) {
   SplitPick best{1, pick_tile_cols(m, n, k, 1, ctas, gate_up)};
   if (gate_up) return best;
   double cost = tile_cost(m, n, k, 1, ctas, best.cols, false) * (1.0 - kMargin);
   for (int split = 2; split <= 4; split *= 2) {
+    if ((k + 63) / 64 < 4 * split) continue;
     // fours do not fill a GPC of the chip whose SMs are no multiple of four: leave some room
-    const long long room = split == 4 ? ctas - ctas / 8 : ctas;
-    for (int bn = kMaxTileCols; bn >= kTileColStep * split; bn -= kTileColStep * split) {
-      const long long tiles = (m + 127) / 128 * ((n + bn - 1) / bn);
-      if (tiles * split > room || (k + 63) / 64 < 4 * split) continue;
-      const double c = tile_cost(m, n, k, 1, ctas, bn, false, split);
-      if (c < cost) { cost = c; best = {split, bn}; }
-    }
+    const int room = split == 4 ? ctas - ctas / 8 : ctas;
+    double c = 0.0;
+    const int bn = pick_split_cols(m, n, k, room, split, &c);
+    if (bn != 0 && c < cost) { cost = c; best = {split, bn}; }
   }
   return best;
 }

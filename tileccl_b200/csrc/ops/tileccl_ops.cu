@@ -266,8 +266,9 @@ int tcl_gemm_smem_bytes(int cta_group) {
 }
 
 int tcl_gemm_pick_tile(int64_t m, int64_t n, int64_t k, int cta_group, int ctas, int gate_up) {
-  return pick_cols(m, n, k, cta_group, ctas, gate_up != 0);
+  return cta_group == 1 ? pick_split(m, n, k, ctas, gate_up != 0).cols : pick_cols(m, n, k, cta_group, ctas, gate_up != 0);
 }
+int tcl_gemm_pick_split(int64_t m, int64_t n, int64_t k, int ctas) { return pick_split(m, n, k, ctas, false).split; }
 int tcl_gemm_pick_form(int64_t m, int64_t n, int64_t k, int ctas) { return pick_cta_group(m, n, k, ctas); }
 int tcl_gemm_plan_split(void* plan) { return plan ? static_cast<GemmPlan*>(plan)->params.split : 0; }
 int tcl_gemm_plan_tile_cols(void* plan) { return plan ? static_cast<GemmPlan*>(plan)->params.bn * static_cast<GemmPlan*>(plan)->params.halves : 0; }
@@ -383,10 +384,16 @@ void* tcl_gemm_plan_create(const tcl_gemm_desc* d, char* err, int errlen) {
   int cols = local ? pick_cols(d->M, d->N, d->K, G, grid, d->epi_silu_mul != 0) : kMaxTileCols;
   const bool split_ok = local && G == 1 && !d->epi_silu_mul && !d->epi_st256 && !d->ablate;
   p.split = 1;
-  if (split_ok && d->split_k == 0 && d->tile_cols == 0) {
-    const SplitPick s = pick_split(d->M, d->N, d->K, grid, false);
-    p.split = s.split;
-    cols = s.cols;
+  if (split_ok && d->tile_cols == 0) {
+    if (d->split_k == 0) {
+      const SplitPick s = pick_split(d->M, d->N, d->K, grid, false);
+      p.split = s.split;
+      cols = s.cols;
+    } else if (d->split_k == 2 || d->split_k == 4) {
+      double cost = 0.0;
+      const int fit = pick_split_cols(d->M, d->N, d->K, grid, d->split_k, &cost);
+      if (fit != 0) cols = fit;      // else refused below
+    }
   }
   if (d->tile_cols) {
     const bool legal = d->tile_cols == 2 * kMaxTileCols ? wide_ok

@@ -102,9 +102,11 @@ int tcl_gemm_plan_run_on(void* plan, const void* A, const void* B, int epoch, vo
 void tcl_gemm_plan_destroy(void* plan);
 int tcl_gemm_plan_grid(void* plan);
 int tcl_gemm_smem_bytes(int cta_group);
-/* Tile width (columns) that a plan of this shape gets on `ctas` CTAs, the CTA form (1, or 2 with ragged_m where M is an odd
- * multiple of 128) that the estimate prefers, and the width a plan has. */
+/* By estimate, for a single-rank plan of this shape on `ctas` CTAs: its tile width in columns, the CTAs that share a tile's K
+ * in the one-CTA form (with gate_up always 1), and the CTA form to ask for (1, or 2 with ragged_m where M is an odd multiple
+ * of 128).  Then the width and the split that a plan has. */
 int tcl_gemm_pick_tile(int64_t m, int64_t n, int64_t k, int cta_group, int ctas, int gate_up);
+int tcl_gemm_pick_split(int64_t m, int64_t n, int64_t k, int ctas);
 int tcl_gemm_pick_form(int64_t m, int64_t n, int64_t k, int ctas);
 int tcl_gemm_plan_tile_cols(void* plan);
 int tcl_gemm_plan_split(void* plan);
