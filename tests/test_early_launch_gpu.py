@@ -5,19 +5,25 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
+FORMS = [dict(cta_group=1), dict(cta_group=1, tile_cols=64), dict(cta_group=1, tile_cols=128, split_k=2), dict(cta_group=1, tile_cols=128, split_k=4),
+         dict(cta_group=2, tile_cols=256), dict(cta_group=2, tile_cols=96), dict(cta_group=2, tile_cols=512)]
+
+
 @pytest.mark.parametrize("M", [128, 512])
-def test_chains_of_dependent_calls(native_lib, M):
+@pytest.mark.parametrize("form", FORMS, ids=lambda f: "-".join(str(v) for v in f.values()))
+def test_chains_of_dependent_calls(native_lib, M, form):
     """Each call reads what the one before it wrote, another kernel overwrites an input right after the call that
     read it, and results are read by another kernel right after the call that wrote them."""
     from tileccl_b200.ops.gemm import GemmPlan
     torch.manual_seed(M)
     K = 512
+    form = dict(form, ragged_m=form["cta_group"] == 2 and M % 256 != 0)
     w = [torch.randn(K, K, device="cuda", dtype=torch.bfloat16) * K ** -0.5 for _ in range(2)]
     x0 = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
 
     def chain(sync):
         x, y = x0.clone(), torch.empty_like(x0)
-        there, back = GemmPlan(x, w[0], out=y, cta_group=1, timeout_ms=1000), GemmPlan(y, w[1], out=x, cta_group=1, timeout_ms=1000)
+        there, back = GemmPlan(x, w[0], out=y, timeout_ms=1000, **form), GemmPlan(y, w[1], out=x, timeout_ms=1000, **form)
         seen = []
         for i in range(40):
             there()
@@ -39,6 +45,41 @@ def test_chains_of_dependent_calls(native_lib, M):
             torch.cuda.synchronize()
             got = chain(lambda: None)
         assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("tokens,hidden,ffn", [(256, 512, 640), (768, 512, 1024)])
+def test_chain_of_the_fused_pair(native_lib, tokens, hidden, ffn):
+    """All-gather GEMM with the SiLU epilogue, then GEMM + reduce-scatter, its result copied into the next call's input:
+    eager, and from a graph whose kernels count the calls themselves."""
+    from tileccl_b200.models.tp_mlp import TpMlp
+    from tileccl_b200.parallel.heap import SymmetricHeap
+    torch.manual_seed(tokens)
+    x0 = torch.randn(tokens, hidden, device="cuda", dtype=torch.bfloat16)
+    heap = SymmetricHeap(64 << 20)
+    try:
+        eager, graph = (TpMlp(heap, tokens, hidden, ffn, seed=3, init_std=0.05, graph=g) for g in (False, True))
+        graph.capture()
+
+        def chain(call, block, sync):
+            block.x_shard.copy_(x0)
+            seen = []
+            for _ in range(30):
+                y = call()
+                sync()
+                seen.append(y.clone())
+                # behind the call that reads it, ahead of the one that needs it; bounded, so that the feedback cannot grow
+                block.x_shard.copy_(torch.tanh(y) + x0)
+                sync()
+            torch.cuda.synchronize()
+            block.check()
+            return torch.stack(seen)
+
+        want = chain(eager, eager, torch.cuda.synchronize)
+        assert torch.isfinite(want).all()
+        assert torch.equal(chain(eager, eager, lambda: None), want)
+        assert torch.equal(chain(graph.replay, graph, lambda: None), want)
+    finally:
+        heap.close()
 
 
 @pytest.mark.parametrize("cta_group", [1, 2])
