@@ -514,8 +514,9 @@ void* tcl_gemm_plan_create(const tcl_gemm_desc* d, char* err, int errlen) {
   pl->cta_group = G;
   // Not across ranks: there CTAs wait for other CTAs and ranks, and an early CTA would hold an SM that they may need.  Not
   // with a grid cap either: its caller has given the other SMs away, and a call that waits beside the one before it
-  // would hold twice the cap.
-  p.early_dependents = local && !d->ablate && d->num_ctas <= 0;
+  // would hold twice the cap.  A grid that fills the chip sends for the next call at once: 32768 x 28672 x 8192 back to back
+  // takes 11.25 ms so, 11.50 when it waits for its last loads.
+  p.early_dependents = !local || d->ablate || d->num_ctas > 0 ? 0 : grid + G > sms ? 2 : 1;
   pl->lda = d->lda;
   pl->ldb = d->ldb;
   pl->a_ptr = d->A;
