@@ -9,7 +9,9 @@
 //     the issue loop of the producer (240 cycles and 45 for each TMA load: 64 to 160 columns take the same time), or of
 //     the MMA warp, which comes to the same with two loads,
 //     its share of what the L2 delivers to all active CTAs (10000 bytes a cycle, 95 to one CTA; half of that where K is not
-//     a multiple of 64: 1152 x 2816 x 1000 14.8 us one-CTA, 13.2 in pairs);
+//     a multiple of 64: 1152 x 2816 x 1000 14.8 us one-CTA, 13.2 in pairs.  What counts is rows that do not start on a
+//     128-byte line, and K stands for the pitch of dense operands: an operand with a pitch of its own is judged by its K all
+//     the same);
 //   128 columns of epilogue cost 1700 cycles; the epilogue of one tile overlaps the k-blocks of the next, the last
 //   one's is exposed; a CTA pair starts 2200 cycles later than a single CTA (cluster launch and barriers).
 // A narrower width has to gain more than kMargin: estimates closer than that came out either way from one board to the
@@ -116,7 +118,10 @@ inline int pick_cta_group(long long m, long long n, long long k, int ctas) {
 // less from the L2 than 256 x 256, but both accumulator buffers belong to one item and its epilogue is hidden only by
 // the skew at its ends.  Sustained, us, 256 against 512 columns: 8192^3 885 -> 843, 16384 x 7168 x 8192 1581 -> 1465,
 // 32768 x 28672 x 8192 13.3 -> 12.5 ms, 16384 x 8192 x 3584 758 -> 738, but K = 1024 (32768 x 8192) 453 -> 470, and with 2.2
-// waves of items (4992 x 4096 x 4096) 141 -> 145.
+// waves of items (4992 x 4096 x 4096) 141 -> 145.  Around the two lines, each width run alone until its clock settled: 16384 x
+// 8192 with K = 1536 320 -> 330, 2048 421 -> 422, 2560 520 -> 516, 3072 619 -> 611, 3584 718 -> 709; with K = 4096 and 3.5 waves
+// (4096 x 8192) 208 -> 208, 4.3 waves 263 -> 267, 6.9 waves 413 -> 406; with K = 8192 and 2.6 waves 333 -> 325, 3.5 waves 419 -> 411,
+// 4.3 waves 533 -> 517.  The lines lie inside the band where the two differ by under 3 %.
 constexpr int kWideMinK = 3072;
 constexpr int kWideMinWaves = 4;
 // Raster group of wide tiles, in tile rows: 16 x 256 rows by 4.6 x 512 columns is what 74 pairs work on at a time, nearer

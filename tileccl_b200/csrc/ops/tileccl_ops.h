@@ -94,7 +94,8 @@ void* tcl_gemm_plan_create(const tcl_gemm_desc* d, char* err, int errlen);
 int tcl_gemm_plan_run(void* plan, int epoch, void* stream);
 /* Points the plan at other A / B operands of the same shape, pitch and alignment (re-encodes the two tensor
  * maps on the host; no device work).  Takes effect for launches made after it returns; not safe while another
- * thread launches the same plan.  For TCL_MODE_AG_GEMM, A is the gathered buffer and must stay what it was. */
+ * thread launches the same plan.  For TCL_MODE_AG_GEMM, A is the gathered buffer and must stay what it was.  For operands that
+ * change from call to call tcl_gemm_plan_run_on is one call instead of two. */
 int tcl_gemm_plan_set_operands(void* plan, const void* A, const void* B);
 /* One launch on other operands of the plan's layout; the plan itself is not changed, so that several threads may do
  * this at once.  With AG+GEMM across ranks A has to be the plan's gathered buffer; on one rank it may be any. */

@@ -9,9 +9,6 @@ from .. import _native
 from ._plan import raw_stream
 
 
-_stream_ptr = raw_stream
-
-
 def silu_mul(gate_up: torch.Tensor, out: torch.Tensor | None = None, stream=None) -> torch.Tensor:
     """``silu(gate_up[:, :F]) * gate_up[:, F:]`` for a contiguous bf16 [rows, 2F] input."""
     if gate_up.dtype != torch.bfloat16 or not gate_up.is_contiguous() or gate_up.dim() != 2:
@@ -20,7 +17,7 @@ def silu_mul(gate_up: torch.Tensor, out: torch.Tensor | None = None, stream=None
     f = two_f // 2
     if out is None:
         out = torch.empty(rows, f, dtype=torch.bfloat16, device=gate_up.device)
-    _native.check(_native.lib().tcl_silu_mul(gate_up.data_ptr(), out.data_ptr(), rows, f, _stream_ptr(stream)), "silu_mul")
+    _native.check(_native.lib().tcl_silu_mul(gate_up.data_ptr(), out.data_ptr(), rows, f, raw_stream(stream)), "silu_mul")
     return out
 
 
@@ -28,7 +25,7 @@ def fill_normal_(t: torch.Tensor, seed: int, mean: float = 0.0, std: float = 1.0
     """In-place N(mean, std) fill of a contiguous bf16 tensor (counter-based, reproducible)."""
     if t.dtype != torch.bfloat16 or not t.is_contiguous():
         raise ValueError("fill_normal_ wants a contiguous bf16 tensor")
-    _native.check(_native.lib().tcl_fill_normal_bf16(t.data_ptr(), t.numel(), seed, mean, std, _stream_ptr(stream)), "fill")
+    _native.check(_native.lib().tcl_fill_normal_bf16(t.data_ptr(), t.numel(), seed, mean, std, raw_stream(stream)), "fill")
     return t
 
 
@@ -41,7 +38,7 @@ def max_rel_err(got: torch.Tensor, ref_f32: torch.Tensor, stream=None) -> float:
     scratch = torch.empty(1024, dtype=torch.float32, device=got.device)
     res = torch.empty(1, dtype=torch.float32, device=got.device)
     _native.check(_native.lib().tcl_max_rel_err(got.data_ptr(), ref_f32.data_ptr(), got.numel(),
-                                                scratch.data_ptr(), res.data_ptr(), _stream_ptr(stream)), "verify")
+                                                scratch.data_ptr(), res.data_ptr(), raw_stream(stream)), "verify")
     return float(res.item())
 
 
@@ -69,10 +66,10 @@ class DeviceBarrier:
         self.epoch += 1
         if self.transport == "nvls":
             _native.check(_native.lib().tcl_barrier_all_mc(self.mc_ptr, self.counter.data_ptr(), self.heap.world, self.heap.rank, self.epoch,
-                                                           self.status.data_ptr(), self.timeout_ns, _stream_ptr(stream)), "barrier")
+                                                           self.status.data_ptr(), self.timeout_ns, raw_stream(stream)), "barrier")
             return
         _native.check(_native.lib().tcl_barrier_all(self.ptrs, self.heap.world, self.heap.rank, self.epoch,
-                                                    self.status.data_ptr(), self.timeout_ns, _stream_ptr(stream)), "barrier")
+                                                    self.status.data_ptr(), self.timeout_ns, raw_stream(stream)), "barrier")
 
     def check(self) -> None:
         st = self.status.tolist()

@@ -66,7 +66,7 @@ class GemmPlan(Plan):
         d.tile_cols = tile_cols
         d.split_k = split_k
         d.comm_form = 1 if (bool(dst_ptrs) if comm_form is None else comm_form) else 0
-        # hold_operands=False: the caller re-points the plan with set_operands() and owns the operands' lifetime
+        # hold_operands=False: the caller names the operands of every launch (run_on) and owns their lifetime
         super().__init__(d, keep_alive=(A, Bt, out) if hold_operands else (out,))
         self.out = out
 

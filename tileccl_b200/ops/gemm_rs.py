@@ -100,7 +100,7 @@ class GemmRs:
         d.ragged_m = 1 if ragged_m else 0
         d.comm_form = 1 if comm_form else 0    # on one rank: the kernel form that several ranks have, see GemmPlan
         d.epi_st256 = 1 if st256 else 0    # 32-byte epilogue stores (st.global.v8.b32) instead of 16-byte ones
-        # hold_operands=False: the caller re-points the plan with plan.set_operands() and owns the operands' lifetime
+        # hold_operands=False: the caller names the operands of every launch (plan.run_on) and owns their lifetime
         own = (self.stage, self.tile_cnt, self.barrier, self.out)
         self.plan = Plan(d, keep_alive=((A, Bt) + own) if hold_operands else own, device_epoch=device_epoch)
         self.rs_chunks = rs_chunks

@@ -9,14 +9,20 @@
     torch.ops.tileccl.barrier()                      # device barrier over all ranks, on the current stream
 
 Plans (tensor maps, staging buffers, counters) are built on first use for a given operand *layout* (shapes,
-row pitches) and are cached; the operands' addresses are not part of the key.  Every call points the cached
-plan at the tensors it was given (a host-side re-encoding of two tensor maps) and keeps no reference to them,
+row pitches) and are cached; the operands' addresses are not part of the key.  Every call launches the cached
+plan on the tensors it was given (a host-side encoding of two tensor maps) and keeps no reference to them,
 so a loop that allocates fresh activations every step reuses one plan and one set of staging buffers, and
 every rank builds the same plans in the same order whatever addresses its allocator hands out.  Results live
 in buffers owned by the cached plan: a result is valid until the next call with operands of the same layout.
-Inputs that must be peer-visible (the AG shard) are copied into the plan's slot of the symmetric heap when
-they are not already there.  Building a fused plan allocates from the symmetric heap and is collective: all
+Across ranks the AG shard must be peer-visible: it is copied into the plan's slot of the symmetric heap when
+it is not already there.  On one rank it is read where it is, if TMA can (dense bf16 on a 16-byte boundary, not
+overlapping the result).  Building a fused plan allocates from the symmetric heap and is collective: all
 ranks must make the same sequence of first calls.
+
+A plan repeats its bits exactly, call after call.  On one rank they may depend on the number of rows: problems with few
+tiles split K over two or four CTAs, which add their fp32 partial sums in a fixed order, but another one than an unsplit
+plan (N = K = 4096: M = 128 and 256 split, M = 384 does not).  ``GemmPlan(..., split_k=1)`` and all plans in the pair form
+(``cta_group=2``) add every row's products in the same order whatever M, N and the tile width are.
 
 The reference stops at C++ programs; this layer is what the north star adds.
 """
